@@ -49,26 +49,52 @@ void set_last_error(const std::string& msg);
 // grid has completed and its writes are visible), and the call also lets the
 // next kernel be scheduled. OWL_NO_PDL=1 in the environment launches plainly.
 // ----------------------------------------------------------------------------
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_prologue() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pdl_trigger();
+    pdl_wait();
+}
+
+// barrier over the CTAs of a thread-block cluster: what every thread wrote
+// before it (global or shared memory) is visible to every thread after it
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 bool pdl_enabled();
 
+// cluster: dimensions of the thread-block clusters
 template <typename... KArgs, typename... Args>
-void launch_pdl(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
+void launch_pdl_cluster(void (*k)(KArgs...), dim3 grid, dim3 block, dim3 cluster, size_t smem, cudaStream_t s,
+                        Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (cluster.x * cluster.y * cluster.z > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = cluster.x;
+        attr[n].val.clusterDim.y = cluster.y;
+        attr[n].val.clusterDim.z = cluster.z;
+        ++n;
+    }
+    if (pdl_enabled()) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n].val.programmaticStreamSerializationAllowed = 1;
+        ++n;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = pdl_enabled() ? 1 : 0;
+    cfg.numAttrs = n;
     OWL_CUDA(cudaLaunchKernelEx(&cfg, k, static_cast<KArgs>(args)...));
+}
+template <typename... KArgs, typename... Args>
+void launch_pdl(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
+    launch_pdl_cluster(k, grid, block, dim3(1, 1, 1), smem, s, args...);
 }
 
 // ----------------------------------------------------------------------------
@@ -141,14 +167,26 @@ struct HostCSR {
     int ntaps() const { return (int)field.size(); }
 };
 
+// a tap as the point kernels read it: one 16-byte load
+struct alignas(16) TapRec {
+    long long off;  // offset inside one shot's field
+    int fi;         // field slot, or the item (trace) for scatter tables
+    float w;
+};
+
 struct DevCSR {
     DevBuf<int> ptr, field, shot, item;
     DevBuf<long long> off;
     DevBuf<float> w;
+    DevBuf<TapRec> tap;
     int nitems = 0, ntaps = 0;
-    void upload(const HostCSR& h, cudaStream_t s) {
+    // by_item: the packed taps carry the item instead of the field
+    void upload(const HostCSR& h, cudaStream_t s, bool by_item = false) {
         nitems = h.nitems();
         ntaps = h.ntaps();
+        std::vector<TapRec> t(ntaps);
+        for (int j = 0; j < ntaps; ++j) t[j] = TapRec{h.off[j], by_item ? h.item[j] : h.field[j], h.w[j]};
+        tap.upload(t.data(), t.size(), s);
         ptr.upload(h.ptr.data(), h.ptr.size(), s);
         field.upload(h.field.data(), h.field.size(), s);
         shot.upload(h.shot.data(), h.shot.size(), s);
@@ -166,11 +204,12 @@ struct CSRView {
     const int* item;
     const long long* off;
     const float* w;
+    const TapRec* tap;
     int nitems;
 };
 
 inline CSRView view(const DevCSR& d) {
-    return CSRView{d.ptr.p, d.field.p, d.shot.p, d.item.p, d.off.p, d.w.p, d.nitems};
+    return CSRView{d.ptr.p, d.field.p, d.shot.p, d.item.p, d.off.p, d.w.p, d.tap.p, d.nitems};
 }
 
 // FD coefficients of the optimised staggered scheme (src/lib/module_fdcoef.f90:23-30, 59-62)

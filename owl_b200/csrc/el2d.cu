@@ -1158,14 +1158,8 @@ struct El2dEngine : SsgBase {
         }
         launch_kernel(OWL_K_ADJ_V, S, false);
         launches++;
-        if (nb_sct <= 4) {
-            launch_point_adj(q, S, 1, PA_SCATTER | PA_TICK, stream);
-            launches++;
-        } else {
-            launch_point_adj(q, S, nb_sct, PA_SCATTER, stream);
-            launch_point_adj(q, S, 1, PA_TICK, stream);
-            launches += 2;
-        }
+        launch_point_adj(q, S, nb_sct, PA_SCATTER | PA_TICK, stream);
+        launches++;
     }
 
     // compulsory bytes of one launch: each state / adjoint field read and

@@ -1477,7 +1477,7 @@ struct El3dEngine : SsgBase {
     }
     int step_launches(int kind) const override {
         if (kind != 2) return SsgBase::step_launches(kind);
-        return 2 + (want_src_now ? 1 : 0) + (nb_sct <= 4 ? 1 : 2);
+        return 3 + (want_src_now ? 1 : 0);
     }
     // the z-marching ring kernels (half-width 4); MP: M-PML coefficients per shell node
     template <bool MP>
@@ -1539,14 +1539,8 @@ struct El3dEngine : SsgBase {
         }
         launch_kernel(OWL_K_ADJ_V, S, false);
         launches++;
-        if (nb_sct <= 4) {
-            launch_point_adj(q, S, 1, PA_SCATTER | PA_TICK, stream);
-            launches++;
-        } else {
-            launch_point_adj(q, S, nb_sct, PA_SCATTER, stream);
-            launch_point_adj(q, S, 1, PA_TICK, stream);
-            launches += 2;
-        }
+        launch_point_adj(q, S, nb_sct, PA_SCATTER | PA_TICK, stream);
+        launches++;
     }
 
     // compulsory bytes per launch (fields once per shot, materials once per

@@ -53,6 +53,7 @@ enum { PT_INJECT = 1, PT_SAMPLE = 2, PT_TICK = 4, PT_NEXT = 8 };  // forward poi
 // advanced by the last CTA, FZ_SCT the residual scatter by extra CTAs of the
 // adjoint velocity-node kernel
 enum { FZ_INJ = 1, FZ_SMP = 2, FZ_TICK = 4, FZ_SCT = 8 };
+constexpr int POINT_CLUSTER = 8;  // most CTAs per shot of a point kernel whose phases meet at a cluster barrier
 constexpr int BOX_W = 9;  // taps of a source along each axis (the 9-tap Kaiser sinc)
 // adjoint point kernel phases. PA_SRC records the source-side adjoint of step
 // t-1 after the scatter; PA_SRC_NOW records that of step t from the fields as
