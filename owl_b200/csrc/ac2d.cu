@@ -520,6 +520,7 @@ __global__ void __launch_bounds__(512) k_ac2d_adj_v(const __grid_constant__ Ac2d
 }
 
 #include "ac2d_vec.cuh"
+#include "ac2d_res.cuh"
 
 // ------------------------- FP64 chain rule ---------------------------------
 // Gradient w.r.t. vp and rho on the padded model grid [-P, n+P+1] from the
@@ -892,6 +893,11 @@ struct Ac2dEngine : SsgBase {
     DevBuf<unsigned> pbar;  // the grid barrier's arrival count and generation
     int num_sms = 0;
     bool run_steps_persistent(int kind, int n, int S) override {
+        if (kind != 2 && resident(0, S)) {
+            if (R == 4) launch_res<4>(kind, n, S);
+            else launch_res<8>(kind, n, S);
+            return true;
+        }
         const char* e = std::getenv("OWL_PERSIST");
         if (!(e && e[0] == '1' && e[1] == 0) || kind == 2 || !fuse_fwd || tz_f < 100 || tz_f >= 200) return false;
         if (R == 4) return persist_r<4>(kind, n, S);
@@ -939,6 +945,168 @@ struct Ac2dEngine : SsgBase {
         OWL_CUDA(cudaLaunchCooperativeKernel((void*)k, dim3(nblocks), dim3(32, ty), args, 0, stream));
         launches += 1;
         return true;
+    }
+
+    // ---- segments with the state resident in shared memory (ac2d_res.cuh) ----
+    struct ResPlan {
+        bool ok = false;
+        Ac2dRes q{};
+        size_t smem = 0;
+        int threads = 0, H = 4;
+        bool one = true;
+        double us = 0.0;  // modelled time of a step of the whole batch
+    };
+    std::map<int, ResPlan> res_plans;  // by shots per launch
+    // rows of each CTA. The slowest CTA sets the pace, and a z-PML row costs about
+    // 1.4 times an interior one, so the rows are split by that weight: the least
+    // common limit that holds all rows, no CTA above its shared memory or, where
+    // that is possible, above the rows that its threads take in one pass; in
+    // multiples of a thread's rows, since a ragged last item costs a whole one.
+    bool res_split(int C, Ac2dRes& q, size_t& smem) const {
+        const bool fsf = desc.free_surface != 0;
+        const int rows = R + NZp - q.zlo;
+        q.C = C;
+        if (rows < C * (R + 1)) return false;
+        std::vector<int> npi(rows + 1, 0), nph(rows + 1, 0);  // z-PML rows above row l
+        for (int l = 0; l < rows; ++l) {
+            const int z = q.zlo + l;
+            npi[l + 1] = npi[l] + ((!fsf && z < pr) || z >= pr + nz);
+            nph[l + 1] = nph[l] + ((!fsf && z <= pr) || z >= pr + nz);
+        }
+        auto bytes = [&](int l0, int l1) {
+            return sizeof(float) * res_fwd_floats(R, q.XG, q.XP, q.GN, l1 - l0, npi[l1] - npi[l0], nph[l1] - nph[l0]);
+        };
+        const int H = R == 8 ? 2 : 4, cap1 = std::max(R + 1, RES_THREADS / q.XG * H);
+        for (int u = 0; u < 4; ++u) {
+            const int cap = u < 2 ? cap1 : rows, unit = u % 2 ? 1 : H;
+            auto fill = [&](double lim) {
+                int l = 0;
+                for (int r = 0; r < C; ++r) {
+                    q.zb[r] = l;
+                    int e = l;
+                    for (;;) {
+                        const int f = r == C - 1 ? rows : std::min(rows, e + unit);
+                        if (f <= e || f - l > cap || rows - f < (C - 1 - r) * (R + 1) || bytes(l, f) > RES_SMEM) break;
+                        if ((e - l >= R + 1 || r == C - 1) && (f - l) + 0.4 * (npi[f] - npi[l]) > lim) break;
+                        e = f;
+                    }
+                    if (e - l < R + 1) return false;
+                    l = e;
+                }
+                q.zb[C] = l;
+                return l == rows;
+            };
+            double lo = 0.0, hi = 1.5 * rows;
+            if (!fill(hi)) continue;
+            while (hi - lo > 0.2) {
+                const double mid = 0.5 * (lo + hi);
+                (fill(mid) ? hi : lo) = mid;
+            }
+            fill(hi);
+            smem = 0;
+            for (int r = 0; r < C; ++r) smem = std::max(smem, bytes(q.zb[r], q.zb[r + 1]));
+            return true;
+        }
+        return false;
+    }
+
+    // cluster size: the least modelled time of a step of the batch. One CTA per SM
+    // (two on one SM took twice as long as two SMs, and clusters are packed that
+    // way unless the shared memory forbids it), about 2.1 us of barriers and phase
+    // starts per step and 0.41 ns per cell of the largest CTA (measured: 181 x 131
+    // cells on 4 / 8 / 16 CTAs 4.7 / 3.7 / 2.7 us, 441 x 241 on 16 CTAs 5.0 us),
+    // the shots in waves of as many clusters as fit the device. Every fitting size
+    // beats the step launches (8.2 and 8.8 us per step for one shot of these
+    // grids, 35.7 against 25.7 us for 32 shots of the larger).
+    using ResKernel = void (*)(Ac2dDev, Ac2dRes);
+    template <int RR>
+    static ResKernel res_kernel(int H, bool store, bool one) {
+        if (RR == 4 && H == 4)
+            return store ? (one ? k_ac2d_fwd_res<4, 4, true, true> : k_ac2d_fwd_res<4, 4, true, false>)
+                         : (one ? k_ac2d_fwd_res<4, 4, false, true> : k_ac2d_fwd_res<4, 4, false, false>);
+        return store ? (one ? k_ac2d_fwd_res<RR, 2, true, true> : k_ac2d_fwd_res<RR, 2, true, false>)
+                     : (one ? k_ac2d_fwd_res<RR, 2, false, true> : k_ac2d_fwd_res<RR, 2, false, false>);
+    }
+    template <int RR>
+    const ResPlan& res_plan(int S) {
+        auto it = res_plans.find(S);
+        if (it != res_plans.end()) return it->second;
+        ResPlan best;
+        for (int v = 0; v < 8; ++v) {
+            auto f = res_kernel<RR>(v & 1 ? 4 : 2, v & 2, v & 4);
+            OWL_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            OWL_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RES_SMEM));
+        }
+        for (int C = 1; C <= RES_MAXC; C *= 2) {
+            ResPlan p;
+            Ac2dRes& q = p.q;
+            q.XG = (NXp + 3) / 4;
+            q.XP = 4 * q.XG + 2 * R;
+            q.GL = (P + 1 + 3) / 4;              // x <= pr: columns 0 .. P
+            q.GR = std::max(q.GL, (P + nx) / 4);  // x >= pr + nx: columns P + nx ..
+            q.GN = q.GL + q.XG - q.GR;
+            q.zlo = desc.free_surface ? pr : R;
+            if (!res_split(C, q, p.smem)) continue;
+            int rows = 0;
+            for (int r = 0; r < C; ++r) rows = std::max(rows, q.zb[r + 1] - q.zb[r]);
+            // rows per thread: two while the CTA's threads suffice (a shorter chain per
+            // phase) and always at half-width 8 (registers), else four (fewer reads)
+            auto items_of = [&](int H) { return q.XG * ((rows + H - 1) / H); };
+            p.H = RR == 8 || items_of(2) <= RES_THREADS ? 2 : 4;
+            const int items = items_of(p.H);
+            const int passes = (items + RES_THREADS - 1) / RES_THREADS;
+            p.one = passes == 1;
+            p.threads = std::max(128, ((items + passes - 1) / passes + 31) / 32 * 32);
+            p.smem = std::max(p.smem, RES_SMEM / 2 + 1024);  // one CTA per SM
+            cudaLaunchConfig_t cfg = {};
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = C; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+            cfg.attrs = at; cfg.numAttrs = 1;
+            cfg.gridDim = dim3(C, S);
+            cfg.blockDim = dim3(p.threads);
+            cfg.dynamicSmemBytes = p.smem;
+            int slots = 0;
+            if (cudaOccupancyMaxActiveClusters(&slots, res_kernel<RR>(p.H, true, p.one), &cfg) != cudaSuccess || slots < 1) {
+                (void)cudaGetLastError();
+                continue;
+            }
+            const int waves = (S + slots - 1) / slots;
+            p.us = waves * (4.1e-4 * rows * NXp + 2.1);
+            p.ok = true;
+            if (!best.ok || p.us < best.us) best = p;
+        }
+        return res_plans[S] = best;
+    }
+    // forward steps of the batch run resident: the automatic mode, explosion
+    // sources only (force taps enter between the velocity update and the halo
+    // exchange), traces that the threads of one CTA can hold
+    bool resident(int pass, int S) override {
+        if (pass != 0 || !res_allowed || fuse_fwd || (inj_fmask & 6)) return false;
+        const ResPlan& p = R == 4 ? res_plan<4>(S) : res_plan<8>(S);
+        return p.ok && max_traces <= 2 * p.threads;
+    }
+    template <int RR>
+    void launch_res(int kind, int n, int S) {
+        const ResPlan& p = res_plan<RR>(S);
+        Ac2dDev a = dev(S);
+        Ac2dRes q = p.q;
+        q.n = n;
+        q.smp = kind != 1;
+        q.inj_last = inj_last.p;
+        const bool store = kind == 1 || kind == 3;
+        const ResKernel k = res_kernel<RR>(p.H, store, p.one);
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = q.C; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+        cfg.attrs = at; cfg.numAttrs = 1;
+        cfg.gridDim = dim3(q.C, S);
+        cfg.blockDim = dim3(p.threads);
+        cfg.dynamicSmemBytes = p.smem;
+        cfg.stream = stream;
+        OWL_CUDA(cudaLaunchKernelEx(&cfg, k, a, q));
+        launches++;
     }
 
     // compulsory bytes of one launch (each state field read / written once per

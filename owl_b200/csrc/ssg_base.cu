@@ -451,6 +451,13 @@ void SsgBase::build_tables(int S, const owl_shot* shots, bool need_sct) {
         hrec_ptr.push_back(rtot);
         hsct_ptr.push_back(hsct.nitems());
     }
+    // the last step with a nonzero amplitude, per shot
+    std::vector<int> hlast(std::max(S, 1), 0);
+    for (int s = 0; s < S; ++s)
+        for (int it = hinj_ptr[s]; it < hinj_ptr[s + 1]; ++it)
+            for (int t = nt; t > hlast[s]; --t)
+                if (hamp[(size_t)it * nt + t - 1] != 0.f) hlast[s] = t;
+    inj_last.upload(hlast.data(), hlast.size(), stream);
     int mr = 0, ms = 0;
     for (size_t i = 0; i + 1 < hrec_ptr.size(); ++i) mr = std::max(mr, hrec_ptr[i + 1] - hrec_ptr[i]);
     for (size_t i = 0; i + 1 < hsct_ptr.size(); ++i) ms = std::max(ms, hsct_ptr[i + 1] - hsct_ptr[i]);
@@ -459,6 +466,7 @@ void SsgBase::build_tables(int S, const owl_shot* shots, bool need_sct) {
         const int b = std::max(1, std::min(1024, (n + 255) / 256));
         return b > POINT_CLUSTER ? b : b > 4 ? POINT_CLUSTER : b > 2 ? 4 : b;
     };
+    max_traces = mr;
     nb_rec = ctas(mr);
     nb_sct = ctas(ms);
     inj.upload(hinj, stream);
@@ -701,6 +709,7 @@ void SsgBase::resolve_opts(const owl_run_opts& o, int nshots, const owl_shot* sh
     plan_B = B;
     spt_f = spt_a = std::min(o.shots_per_cta > 0 ? o.shots_per_cta : 1, B);
     graph = o.use_graph >= 0;
+    res_allowed = tune && graph;
     launch_params(o);
 }
 
@@ -725,31 +734,30 @@ std::vector<int> SsgBase::tune_tz(int pass) const {
     return {4, 8, 16};
 }
 
-void SsgBase::autotune(int S, int k, bool grad) {
-    auto key = std::make_pair(S, grad ? 1 : 0);
-    auto it = tune_cache.find(key);
-    if (it != tune_cache.end()) {
-        spt_f = it->second[0]; tz_f = it->second[1]; spt_a = it->second[2]; tz_a = it->second[3];
-        tune_extra(S, k, grad);
-        return;
-    }
-    cur_k = k;
-    set_step(k);
+void SsgBase::autotune(int S, int k, bool grad, bool all) {
     // the forward pass's choice is shared by the forward-only and the gradient
     // entries of S: the forwards of a misfit and of a gradient of one handle
     // run the same kernels (their seismograms equal to the bit)
-    const auto other = tune_cache.find(std::make_pair(S, grad ? 0 : 1));
-    const bool have_fwd = other != tune_cache.end();
-    if (have_fwd) { spt_f = other->second[0]; tz_f = other->second[1]; }
+    cur_k = k;
     for (int pass = 0; pass < (grad ? 2 : 1); ++pass) {
-        if (pass == 0 && have_fwd) continue;
+        int& spt_x = pass == 0 ? spt_f : spt_a;
+        int& tz_x = pass == 0 ? tz_f : tz_a;
+        const auto it = tune_cache.find(std::make_pair(S, pass));
+        if (it != tune_cache.end()) {
+            spt_x = it->second[0];
+            tz_x = it->second[1];
+            continue;
+        }
+        if (!all && resident(pass, S)) continue;
+        set_step(k);
         const std::vector<int> tzs = tune_tz(pass);
         float best = 1e30f;
         int bs = 1, bt = tzs[std::min<size_t>(1, tzs.size() - 1)];
         for (int spt : tune_spt(pass)) {
             if (spt > S) break;
             for (int tz : tzs) {
-                if (pass == 0) { spt_f = spt; tz_f = tz; } else { spt_a = spt; tz_a = tz; }
+                spt_x = spt;
+                tz_x = tz;
                 // the forward variants the time loop launches (the fused injection,
                 // without the sampling CTAs and the step counter); the adjoint's
                 // fused work is the residual scatter of extra CTAs, whose residual
@@ -775,9 +783,10 @@ void SsgBase::autotune(int S, int k, bool grad) {
                 if (ms < best) { best = ms; bs = spt; bt = tz; }
             }
         }
-        if (pass == 0) { spt_f = bs; tz_f = bt; } else { spt_a = bs; tz_a = bt; }
+        spt_x = bs;
+        tz_x = bt;
+        tune_cache[std::make_pair(S, pass)] = {bs, bt};
     }
-    tune_cache[key] = {spt_f, tz_f, spt_a, tz_a};
     tune_extra(S, k, grad);
 }
 
@@ -829,6 +838,10 @@ void SsgBase::forward_batch(int S, int k, bool graph, bool save, bool store_last
     launch_point_fwd(q, S, nb_rec, PT_SAMPLE, stream);
     OWL_LAUNCH_CHECK();
     launches++;
+    if (!save && resident(0, S)) {
+        run_steps(0, nt, S, q, graph);  // no checkpoints: one segment
+        return;
+    }
     const int nseg = (nt + k - 1) / k;
     for (int sg = 0; sg < nseg; ++sg) {
         const bool last = store_last && sg == nseg - 1;
@@ -1240,6 +1253,8 @@ void SsgBase::kernel_time(int id, int nlaunch, double* avg_ms, double* bytes) {
     OWL_CHECK((kid < OWL_K_ADJ_P && !store) ||
                   (ad.p && G.p && Sbuf.p && ad.n >= (size_t)sad * S && Sbuf.n >= (size_t)nS * cur_k * S * fs),
               OWL_ERR_INVALID, "adjoint kernels and store variants need a gradient call first");
+    // (a handle whose segments ran resident has not tuned the step kernels yet)
+    if (tune) autotune(S, cur_k, ad.p && G.p && ad.n >= (size_t)sad * S && Sbuf.n >= (size_t)nS * cur_k * S * fs, true);
     set_step(cur_k);
     // the variant the time loop launches, without advancing the step counter
     const int fz = kid < OWL_K_ADJ_P ? (fuse_fwd ? FZ_INJ : 0) : (fuse_on ? FZ_SCT : 0);

@@ -108,6 +108,9 @@ struct SsgBase : Engine {
     int inj_fmask = 0;     // fields the batch's sources inject into (bit f: field f)
     bool want_src_now = false;  // the adjoint sweep records the source-side adjoint
     int fz_mode = 0;       // FZ_* work of the next stencil launches
+    bool res_allowed = false;  // this call may run whole segments as one launch (automatic tiles, graphs on)
+    int max_traces = 0;        // most traces of a shot of the batch
+    DevBuf<int> inj_last;      // per shot: last step (1-based) whose source amplitudes are not all zero
     DevBuf<unsigned char> live;
     DevBuf<long long> segbuf;  // st_segments offsets then lengths, on the device
     GraphCache g_fwd, g_rec, g_adj, g_fst;
@@ -122,7 +125,7 @@ struct SsgBase : Engine {
     std::vector<int> item_src, item_comp, item_shot;
     std::vector<long long> item_rho_cell;  // padded-grid index of the rho scaling a force component, -1 otherwise
     std::vector<float> item_rho;
-    std::map<std::pair<int, int>, std::array<int, 4>> tune_cache;
+    std::map<std::pair<int, int>, std::array<int, 2>> tune_cache;  // (S, pass) -> shots per CTA, tile
     std::vector<float> h_rhop;  // padded rho, storage layout (force-source weights)
     std::vector<int> h_gather_ptr;  // trace ranges of the (shot, component) gathers of the batch
     AdjointSource adjsrc;
@@ -210,6 +213,12 @@ struct SsgBase : Engine {
         (void)kind; (void)n; (void)S;
         return false;
     }
+    // whether the medium runs the forward (pass 0) / adjoint (pass 1) steps of a
+    // batch of S shots as one launch per segment (automatic mode)
+    virtual bool resident(int pass, int S) {
+        (void)pass; (void)S;
+        return false;
+    }
     void run_steps(int kind, int n, int S, const PointDev& q, bool graph);
     void resolve_opts(const owl_run_opts& o, int nshots, const owl_shot* shots, bool grad, int& B, int& k,
                       bool& graph);
@@ -218,7 +227,8 @@ struct SsgBase : Engine {
     // bytes of the buffers a new batch would reuse or replace
     double held_bytes() const;
     int plan_k = 0, plan_B = 0;  // the last call's checkpoint interval and shots per batch
-    void autotune(int S, int k, bool grad);
+    // times the tile candidates of the passes that run step by step (all: of both passes)
+    void autotune(int S, int k, bool grad, bool all = false);
     void save_ckpt(int slot, int S);
     void restore_ckpt(int slot, int S);
     void forward_batch(int S, int k, bool graph, bool save, bool store_last = false);
