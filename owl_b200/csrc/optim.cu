@@ -27,73 +27,179 @@ namespace {
 
 constexpr int RED_BLOCKS = 148 * 8;
 
-// partial sums of up to three products per block: (s.q, y.s, y.y) with
-// s = x1 - x0 (or x1 alone), y = g1 - g0 (or g1 alone), q
-__global__ void __launch_bounds__(256) k_dots(long long n, const float* __restrict__ x1, const float* __restrict__ x0,
-                                              const float* __restrict__ g1, const float* __restrict__ g0,
-                                              const float* __restrict__ q, double* __restrict__ part) {
-    double a = 0.0, b = 0.0, c = 0.0;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const double s = x1 ? (double)x1[i] - (x0 ? (double)x0[i] : 0.0) : 0.0;
-        const double y = (double)g1[i] - (g0 ? (double)g0[i] : 0.0);
-        const double qq = q ? (double)q[i] : 0.0;
-        a += s * qq;
-        b += y * s;
-        c += y * (q ? qq : y);
-    }
+// ---- search directions as a chain of launches without host round trips ----
+//
+// Each launch of the L-BFGS recursion finishes the dot products of the launch
+// before (every block sums the per-block FP64 partials itself, in a fixed order,
+// so no block waits for another), applies that pair's update to the direction
+// and forms the partials of the next pair in the same pass: 2 np + 1 launches
+// for np pairs, where a dot, a one-thread sum of its partials, a copy to the host
+// and an update per pair were 6 np + 4 launches and 2 np + 1 host waits. A field
+// of 80 k cells is latency bound: 401 x 201, six models, smoothing and taper
+// included, takes 1.6 ms a pass, most of it allocations, against 2.1 ms.
+struct LbStep {
+    long long n;
+    int nparts;               // blocks of the launch before (its partials), 0: none
+    const double* pin;        // nparts x 3 partials
+    double* pout;             // gridDim x 3 partials
+    double* sc;               // alpha[np], ys[np], gamma
+    int np, prev;             // pairs; pair whose dot products pin holds
+    const float* src;         // the direction so far
+    float* r;                 // the direction
+    const float *u1, *u0;     // update vector u1 - u0 of pair prev
+    const float *x1, *x0, *g1, *g0;  // next pair: s = x1 - x0, y = g1 - g0
+};
+enum { LB_FIRST = 0, LB_DOWN, LB_TURN, LB_UP, LB_LAST };
+
+// sums of three values over the block (256 threads, fixed order), in every thread
+__device__ __forceinline__ void block_sum3(double& a, double& b, double& c) {
     __shared__ double red[3][8];
     for (int o = 16; o; o >>= 1) {
         a += __shfl_xor_sync(0xffffffffu, a, o);
         b += __shfl_xor_sync(0xffffffffu, b, o);
         c += __shfl_xor_sync(0xffffffffu, c, o);
     }
-    const int w = threadIdx.x >> 5;
+    __syncthreads();
     if ((threadIdx.x & 31) == 0) {
-        red[0][w] = a;
-        red[1][w] = b;
-        red[2][w] = c;
+        red[0][threadIdx.x >> 5] = a;
+        red[1][threadIdx.x >> 5] = b;
+        red[2][threadIdx.x >> 5] = c;
     }
     __syncthreads();
-    if (threadIdx.x < 3) {
-        double t = 0.0;
-        for (int i = 0; i < 8; ++i) t += red[threadIdx.x][i];
-        part[(size_t)blockIdx.x * 3 + threadIdx.x] = t;
+    a = b = c = 0.0;
+    for (int i = 0; i < 8; ++i) {
+        a += red[0][i];
+        b += red[1][i];
+        c += red[2][i];
+    }
+}
+__device__ __forceinline__ void sum_parts(const double* __restrict__ p, int n, double& a, double& b, double& c) {
+    a = b = c = 0.0;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        a += p[3 * i];
+        b += p[3 * i + 1];
+        c += p[3 * i + 2];
+    }
+    block_sum3(a, b, c);
+}
+
+// MODE: LB_FIRST dots of the newest pair; LB_DOWN q -= alpha y, dots of the next
+// older pair; LB_TURN the oldest pair's q -= alpha y, the scaling gamma, y.r of the
+// oldest pair; LB_UP r += s (alpha - beta), y.r of the next newer pair; LB_LAST the
+// newest pair's update and the sign
+template <int MODE>
+__global__ void __launch_bounds__(256) k_lbfgs(const __grid_constant__ LbStep a) {
+    pdl_prologue();
+    double coef = 0.0, gamma = 0.0;
+    if (MODE != LB_FIRST) {
+        double d0, d1, d2;  // LB_DOWN / LB_TURN: s.q, y.s, y.y (newest pair); LB_UP / LB_LAST: y.r in d2
+        sum_parts(a.pin, a.nparts, d0, d1, d2);
+        double *alpha = a.sc, *ys = a.sc + a.np;
+        if (MODE == LB_DOWN || MODE == LB_TURN) {
+            const double al = d1 == 0.0 ? 0.0 : d0 / d1;
+            coef = -al;
+            if (MODE == LB_TURN) gamma = a.prev == a.np - 1 ? (d2 == 0.0 ? 0.0 : d1 / d2) : a.sc[2 * a.np];
+            if (blockIdx.x == 0 && threadIdx.x == 0) {
+                alpha[a.prev] = al;
+                ys[a.prev] = d1;
+                if (a.prev == a.np - 1) a.sc[2 * a.np] = d2 == 0.0 ? 0.0 : d1 / d2;
+            }
+        } else {
+            const double y = ys[a.prev];
+            coef = alpha[a.prev] - (y == 0.0 ? 0.0 : d2 / y);
+        }
+    }
+    double p0 = 0.0, p1 = 0.0, p2 = 0.0;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += (long long)gridDim.x * blockDim.x) {
+        float q = a.src[i];
+        if (MODE != LB_FIRST) {
+            q = (float)((double)q + coef * ((double)a.u1[i] - (double)a.u0[i]));
+            if (MODE == LB_TURN) q = (float)(gamma * (double)q);
+            if (MODE == LB_LAST) q = -q;
+        }
+        if (MODE != LB_FIRST) a.r[i] = q;
+        if (MODE == LB_LAST) continue;
+        const double y = (double)a.g1[i] - (double)a.g0[i];
+        if (MODE == LB_FIRST || MODE == LB_DOWN) {
+            const double s = (double)a.x1[i] - (double)a.x0[i];
+            p0 += s * (double)q;
+            p1 += y * s;
+            if (MODE == LB_FIRST) p2 += y * y;
+        } else {
+            p2 += y * (double)q;
+        }
+    }
+    if (MODE == LB_LAST) return;
+    block_sum3(p0, p1, p2);
+    if (threadIdx.x == 0) {
+        a.pout[(size_t)blockIdx.x * 3] = p0;
+        a.pout[(size_t)blockIdx.x * 3 + 1] = p1;
+        a.pout[(size_t)blockIdx.x * 3 + 2] = p2;
     }
 }
 
-__global__ void k_sum_parts(const double* __restrict__ part, int nb, double* __restrict__ out) {
-    if (threadIdx.x < 3) {
-        double t = 0.0;
-        for (int i = 0; i < nb; ++i) t += part[(size_t)i * 3 + threadIdx.x];
-        out[threadIdx.x] = t;
-    }
-}
-
-// r = a * r + c * (u1 - u0) [+ d * v]   (u0, v optional)
-// (u1 may be r itself)
-__global__ void k_update(long long n, float* r, double a, double c, const float* u1, const float* __restrict__ u0,
-                         double d, const float* __restrict__ v) {
+// conjugate gradient: partials of gp.gp and (g - gp).g, then the direction
+__global__ void __launch_bounds__(256) k_cg_dots(long long n, const float* __restrict__ g, const float* __restrict__ gp,
+                                                 double* __restrict__ part) {
+    double p0 = 0.0, p1 = 0.0, p2 = 0.0;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        double u = (double)u1[i] - (u0 ? (double)u0[i] : 0.0);
-        double t = (a != 0.0 ? a * (double)r[i] : 0.0) + c * u;  // a = 0: r is write-only
-        if (v) t += d * (double)v[i];
-        r[i] = (float)t;
+        const double v = g[i], w = gp[i];
+        p0 += w * w;
+        p1 += (v - w) * v;
+    }
+    block_sum3(p0, p1, p2);
+    if (threadIdx.x == 0) {
+        part[(size_t)blockIdx.x * 3] = p0;
+        part[(size_t)blockIdx.x * 3 + 1] = p1;
+        part[(size_t)blockIdx.x * 3 + 2] = p2;
     }
 }
+__global__ void __launch_bounds__(256) k_cg_apply(long long n, const double* __restrict__ part, int nparts,
+                                                  const float* __restrict__ g, const float* prev, float* srch) {
+    pdl_prologue();
+    double s1, s2, z;
+    sum_parts(part, nparts, s1, s2, z);
+    const double beta = s1 == 0.0 ? 0.0 : fmax(0.0, s2 / s1);
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+        srch[i] = (float)(-(double)g[i] + beta * (double)prev[i]);
+}
 
-// one axis of a separable filter: field (n1, n2, n3), axis stride `st`, length `len`
-__global__ void k_smooth_axis(const float* __restrict__ in, float* __restrict__ out, long long n, long long st, int len,
-                              const float* __restrict__ w, int rad) {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int p = (int)((i / st) % len);
-        const long long base = i - (long long)p * st;
+__global__ void k_negate(long long n, const float* __restrict__ g, float* __restrict__ r) {
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+        r[i] = -g[i];
+}
+
+// one axis of a separable filter: field (n1, n2, n3), axis stride `st`, length `len`.
+// The weights come in the kernel's parameters (every thread reads the same one:
+// a constant operand), without an upload.
+constexpr int SMOOTH_W = 513;
+struct SmoothW {
+    float w[SMOOTH_W];
+};
+template <typename I>
+__device__ __forceinline__ void smooth_axis(const float* __restrict__ in, float* __restrict__ out, long long n, I st,
+                                            int len, const float* w, int rad) {
+    for (long long ii = (long long)blockIdx.x * blockDim.x + threadIdx.x; ii < n; ii += (long long)gridDim.x * blockDim.x) {
+        const I i = (I)ii;
+        const int p = (int)((i / st) % (I)len);
+        const float* base = in + (ii - (long long)p * (long long)st);
         float acc = 0.f;
         for (int k = -rad; k <= rad; ++k) {
             const int q = min(max(p + k, 0), len - 1);
-            acc += w[k + rad] * in[base + (long long)q * st];
+            acc += w[k + rad] * base[(long long)q * (long long)st];
         }
-        out[i] = acc;
+        out[ii] = acc;
     }
+}
+template <typename I>
+__global__ void k_smooth_axis_p(const float* __restrict__ in, float* __restrict__ out, long long n, I st, int len,
+                                const __grid_constant__ SmoothW w, int rad) {
+    smooth_axis<I>(in, out, n, st, len, w.w, rad);
+}
+// weights of more taps than the parameters hold, from global memory
+__global__ void k_smooth_axis(const float* __restrict__ in, float* __restrict__ out, long long n, long long st, int len,
+                              const float* __restrict__ w, int rad) {
+    smooth_axis<long long>(in, out, n, st, len, w, rad);
 }
 
 __global__ void k_taper(float* __restrict__ f, long long n, int n1, int n2, int n3, int a1, int b1, int a2, int b2,
@@ -214,72 +320,71 @@ __global__ void k_median(const float* __restrict__ in, float* __restrict__ out, 
 
 int blocks_for(long long n) { return (int)std::max<long long>(1, std::min<long long>((n + 255) / 256, RED_BLOCKS)); }
 
-// (s.q, y.s, y.y) on the device, returned to the host
-struct Dots {
-    DevBuf<double> part, out;
-    double v[3];
-    void run(long long n, const float* x1, const float* x0, const float* g1, const float* g0, const float* q,
-             cudaStream_t s) {
-        const int nb = blocks_for(n);
-        part.reserve((size_t)nb * 3);
-        out.reserve(3);
-        k_dots<<<nb, 256, 0, s>>>(n, x1, x0, g1, g0, q, part.p);
-        k_sum_parts<<<1, 32, 0, s>>>(part.p, nb, out.p);
-        OWL_LAUNCH_CHECK();
-        OWL_CUDA(cudaMemcpyAsync(v, out.p, sizeof(v), cudaMemcpyDeviceToHost, s));
-        OWL_CUDA(cudaStreamSynchronize(s));
-    }
-};
-
-void update(long long n, float* r, double a, double c, const float* u1, const float* u0, double d, const float* v,
-            cudaStream_t s) {
-    k_update<<<blocks_for(n), 256, 0, s>>>(n, r, a, c, u1, u0, d, v);
-    OWL_LAUNCH_CHECK();
-}
-
 }  // namespace
 
 // models[0..nm-1] oldest first, grads alike; srch written. All device pointers.
 void search_direction(int method, long long n, int nm, const float* const* x, const float* const* g,
                       const float* prev_srch, float* srch, cudaStream_t s) {
-    Dots dots;
     const float* gk = g[nm - 1];
+    // two blocks per SM at most: every launch sums the partials of the one before
+    const int nb = (int)std::max<long long>(1, std::min<long long>((n + 255) / 256, 2 * 148));
     if (method == OWL_SEARCH_SD || nm < 2) {
-        update(n, srch, 0.0, -1.0, gk, nullptr, 0.0, nullptr, s);
+        k_negate<<<nb, 256, 0, s>>>(n, gk, srch);
+        OWL_LAUNCH_CHECK();
         return;
     }
+    const int np = nm - 1;
+    DevBuf<double> wbuf;  // two sets of partials, then alpha, ys, gamma
+    wbuf.reserve((size_t)6 * nb + 2 * np + 1);
+    double* work = wbuf.p;
     if (method == OWL_SEARCH_CG) {
         // Polak-Ribiere: beta = max(0, g.(g - gp) / gp.gp), srch = -g + beta srch_prev
         OWL_CHECK(prev_srch, OWL_ERR_INVALID, "conjugate gradient needs the previous search direction");
-        const float* gp = g[nm - 2];
-        dots.run(n, nullptr, nullptr, gp, nullptr, nullptr, s);
-        const double s1 = dots.v[2];
-        dots.run(n, nullptr, nullptr, gk, gp, gk, s);  // y = g - gp, q = g: c = y.g
-        const double s2 = dots.v[2];
-        const double beta = s1 == 0.0 ? 0.0 : std::max(0.0, s2 / s1);
-        update(n, srch, 0.0, -1.0, gk, nullptr, beta, prev_srch, s);
+        k_cg_dots<<<nb, 256, 0, s>>>(n, gk, g[nm - 2], work);
+        launch_pdl(k_cg_apply, dim3(nb), dim3(256), 0, s, n, (const double*)work, nb, gk, prev_srch, srch);
+        OWL_LAUNCH_CHECK();
+        OWL_CUDA(cudaStreamSynchronize(s));  // the partials are freed on return
         return;
     }
     // L-BFGS two-loop recursion over the pairs (x_{i+1} - x_i, g_{i+1} - g_i), newest first
-    const int np = nm - 1;
-    std::vector<double> alpha(np, 0.0), ys(np, 0.0);
-    OWL_CUDA(cudaMemcpyAsync(srch, gk, n * sizeof(float), cudaMemcpyDeviceToDevice, s));  // q = g_k
-    for (int i = np - 1; i >= 0; --i) {
-        dots.run(n, x[i + 1], x[i], g[i + 1], g[i], srch, s);  // a = s.q, b = y.s
-        ys[i] = dots.v[1];
-        alpha[i] = ys[i] == 0.0 ? 0.0 : dots.v[0] / ys[i];
-        update(n, srch, 1.0, -alpha[i], g[i + 1], g[i], 0.0, nullptr, s);  // q -= alpha y
+    LbStep a{};
+    a.n = n;
+    a.nparts = nb;
+    a.sc = work + (size_t)6 * nb;
+    a.np = np;
+    int flip = 0;
+    auto next_pair = [&](int i) {
+        a.x1 = x[i + 1]; a.x0 = x[i];
+        a.g1 = g[i + 1]; a.g0 = g[i];
+        a.pin = work + (size_t)3 * nb * flip;
+        flip ^= 1;
+        a.pout = work + (size_t)3 * nb * flip;
+    };
+    auto go = [&](void (*k)(LbStep)) { launch_pdl(k, dim3(nb), dim3(256), 0, s, a); };
+    a.src = gk;
+    a.r = srch;
+    next_pair(np - 1);
+    go(k_lbfgs<LB_FIRST>);
+    for (int i = np - 1; i > 0; --i) {  // q -= alpha_i y_i; s.q and y.s of pair i - 1
+        a.prev = i;
+        a.u1 = g[i + 1]; a.u0 = g[i];
+        next_pair(i - 1);
+        go(k_lbfgs<LB_DOWN>);
+        a.src = srch;
     }
-    // initial scaling (s.y) / (y.y) of the newest pair
-    dots.run(n, x[np], x[np - 1], g[np], g[np - 1], nullptr, s);
-    const double gamma = dots.v[2] == 0.0 ? 0.0 : dots.v[1] / dots.v[2];
-    update(n, srch, gamma, 0.0, srch, nullptr, 0.0, nullptr, s);
-    for (int i = 0; i < np; ++i) {
-        dots.run(n, nullptr, nullptr, g[i + 1], g[i], srch, s);  // c = y.r
-        const double beta = ys[i] == 0.0 ? 0.0 : dots.v[2] / ys[i];
-        update(n, srch, 1.0, alpha[i] - beta, x[i + 1], x[i], 0.0, nullptr, s);  // r += s (alpha - beta)
+    a.prev = 0;
+    a.u1 = g[1]; a.u0 = g[0];
+    next_pair(0);
+    go(k_lbfgs<LB_TURN>);
+    a.src = srch;
+    for (int i = 0; i < np; ++i) {  // r += s_i (alpha_i - beta_i); y.r of pair i + 1
+        a.prev = i;
+        a.u1 = x[i + 1]; a.u0 = x[i];
+        next_pair(std::min(i + 1, np - 1));
+        go(i + 1 < np ? k_lbfgs<LB_UP> : k_lbfgs<LB_LAST>);
     }
-    update(n, srch, -1.0, 0.0, srch, nullptr, 0.0, nullptr, s);
+    OWL_LAUNCH_CHECK();
+    OWL_CUDA(cudaStreamSynchronize(s));  // the partials are freed on return
 }
 
 void grad_process(int op, int n1, int n2, int n3, const float* param, const float* mask, float* f, cudaStream_t s) {
@@ -288,10 +393,13 @@ void grad_process(int op, int n1, int n2, int n3, const float* param, const floa
     const int nb = blocks_for(n);
     switch (op) {
         case OWL_GRAD_SMOOTH: {
-            DevBuf<float> tmp, w;
-            tmp.reserve(n);
+            DevBuf<float> w;
+            DevBuf<float> tb;
+            tb.reserve(n);
+            float* tmp = tb.p;
             const int len[3] = {n1, n2, n3};
             const long long st[3] = {1, n1, (long long)n1 * n2};
+            float *cur = f, *other = tmp;  // the axes' passes alternate between the two
             for (int ax = 0; ax < 3; ++ax) {
                 const double sg = param[ax];
                 if (!(sg > 0.0) || len[ax] < 2) continue;
@@ -301,12 +409,25 @@ void grad_process(int op, int n1, int n2, int n3, const float* param, const floa
                 std::vector<double> dw(2 * rad + 1);
                 for (int k = -rad; k <= rad; ++k) tot += dw[k + rad] = std::exp(-0.5 * (double)k * k / (sg * sg));
                 for (int k = 0; k <= 2 * rad; ++k) hw[k] = (float)(dw[k] / tot);
-                w.upload(hw.data(), hw.size(), s);
-                k_smooth_axis<<<nb, 256, 0, s>>>(f, tmp.p, n, st[ax], len[ax], w.p, rad);
-                OWL_LAUNCH_CHECK();
-                OWL_CUDA(cudaMemcpyAsync(f, tmp.p, n * sizeof(float), cudaMemcpyDeviceToDevice, s));
-                OWL_CUDA(cudaStreamSynchronize(s));  // hw is reused by the next axis
+                if (2 * rad + 1 <= SMOOTH_W) {
+                    SmoothW wp;
+                    std::copy(hw.begin(), hw.end(), wp.w);
+                    const int nb1 = (int)std::max<long long>(1, std::min<long long>((n + 255) / 256, 148 * 32));
+                    if (n < (1LL << 31))
+                        k_smooth_axis_p<unsigned><<<nb1, 256, 0, s>>>(cur, other, n, (unsigned)st[ax], len[ax], wp, rad);
+                    else
+                        k_smooth_axis_p<long long><<<nb1, 256, 0, s>>>(cur, other, n, st[ax], len[ax], wp, rad);
+                    OWL_LAUNCH_CHECK();
+                } else {
+                    w.upload(hw.data(), hw.size(), s);
+                    k_smooth_axis<<<nb, 256, 0, s>>>(cur, other, n, st[ax], len[ax], w.p, rad);
+                    OWL_LAUNCH_CHECK();
+                    OWL_CUDA(cudaStreamSynchronize(s));  // w is reused by the next axis
+                }
+                std::swap(cur, other);
             }
+            if (cur != f) OWL_CUDA(cudaMemcpyAsync(f, cur, n * sizeof(float), cudaMemcpyDeviceToDevice, s));
+            OWL_CUDA(cudaStreamSynchronize(s));  // tb is freed on return
             break;
         }
         case OWL_GRAD_TAPER: {
@@ -326,12 +447,13 @@ void grad_process(int op, int n1, int n2, int n3, const float* param, const floa
             OWL_LAUNCH_CHECK();
             break;
         case OWL_GRAD_MAX_BALANCE: {
-            DevBuf<float> part;
-            part.reserve(nb);
-            k_max_part<<<nb, 256, 0, s>>>(f, n, part.p);
+            DevBuf<float> tb;
+            tb.reserve(nb);
+            float* part = tb.p;
+            k_max_part<<<nb, 256, 0, s>>>(f, n, part);
             OWL_LAUNCH_CHECK();
             std::vector<float> hp(nb);
-            OWL_CUDA(cudaMemcpyAsync(hp.data(), part.p, nb * sizeof(float), cudaMemcpyDeviceToHost, s));
+            OWL_CUDA(cudaMemcpyAsync(hp.data(), part, nb * sizeof(float), cudaMemcpyDeviceToHost, s));
             OWL_CUDA(cudaStreamSynchronize(s));
             const float m = *std::max_element(hp.begin(), hp.end());
             if (m != 0.f) {
@@ -341,12 +463,13 @@ void grad_process(int op, int n1, int n2, int n3, const float* param, const floa
             break;
         }
         case OWL_GRAD_RMS_BALANCE: {
-            DevBuf<double> part, tot;
-            part.reserve(1);
-            k_slice_sumsq<<<1, 256, 0, s>>>(f, 1, (int)n, 1, 0, part.p);  // the whole field as one slice
+            DevBuf<double> tb;
+            tb.reserve(1);
+            double* part = tb.p;
+            k_slice_sumsq<<<1, 256, 0, s>>>(f, 1, (int)n, 1, 0, part);  // the whole field as one slice
             OWL_LAUNCH_CHECK();
             double ss = 0.0;
-            OWL_CUDA(cudaMemcpyAsync(&ss, part.p, sizeof(double), cudaMemcpyDeviceToHost, s));
+            OWL_CUDA(cudaMemcpyAsync(&ss, part, sizeof(double), cudaMemcpyDeviceToHost, s));
             OWL_CUDA(cudaStreamSynchronize(s));
             const double rms = std::sqrt(ss / (double)n);
             if (rms != 0.0) {
@@ -392,11 +515,12 @@ void grad_process(int op, int n1, int n2, int n3, const float* param, const floa
             if (n3 == 1) h[2] = 0;
             OWL_CHECK((2 * h[0] + 1) * (2 * h[1] + 1) * (2 * h[2] + 1) <= 343, OWL_ERR_INVALID,
                       "median window above 343 cells");
-            DevBuf<float> tmp;
-            tmp.reserve(n);
-            k_median<<<nb, 256, 0, s>>>(f, tmp.p, n1, n2, n3, h[0], h[1], h[2]);
+            DevBuf<float> tb;
+            tb.reserve(n);
+            float* tmp = tb.p;
+            k_median<<<nb, 256, 0, s>>>(f, tmp, n1, n2, n3, h[0], h[1], h[2]);
             OWL_LAUNCH_CHECK();
-            OWL_CUDA(cudaMemcpyAsync(f, tmp.p, n * sizeof(float), cudaMemcpyDeviceToDevice, s));
+            OWL_CUDA(cudaMemcpyAsync(f, tmp, n * sizeof(float), cudaMemcpyDeviceToDevice, s));
             break;
         }
         default:
