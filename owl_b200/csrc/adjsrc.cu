@@ -739,10 +739,9 @@ void AdjointSource::run(const owl_misfit_opts& o, int ngather, const int* h_gath
                     OWL_CHECK(h_gather_ptr[g + c + 1] - h_gather_ptr[g + c] == h_gather_ptr[g + 1] - h_gather_ptr[g],
                               OWL_ERR_INVALID, "dtw-vector: the component gathers of a shot must hold equal trace counts");
         }
-        DevBuf<double> tmp;
         if (!tm && gm) {
-            tmp.reserve(ntr);
-            tm = tmp.p;
+            ttm.reserve(ntr);
+            tm = ttm.p;
         }
         run_dtw(o, ngather, nt, ntr, syn, obs, adj, tm, tau, s);
         if (gm) {

@@ -13,6 +13,7 @@ struct DftTables {
     int N = 0, M = 0, logM = 0;
     DevBuf<float2> chirp, bf, tw;
     void build(int n, cudaStream_t s);
+    size_t held() const { return sizeof(float2) * (chirp.n + bf.n + tw.n); }
 };
 
 struct AdjointSource {
@@ -25,7 +26,15 @@ struct AdjointSource {
     DevBuf<double> dsn, dob, band, vnrm;  // DTW: normalised traces, per-CTA search bands, receiver norms
     DevBuf<float> qw, warp;         // DTW: quality weights, warped traces
     DevBuf<unsigned short> path;    // DTW: per-CTA back-pointers of the dynamic program
+    DevBuf<float> ttau;             // DTW: shifts, where the caller takes none
+    DevBuf<double> ttm;             // per-trace misfits, where the caller takes only the gathers'
     long long launches = 0;
+    // bytes of device memory held
+    size_t held() const {
+        return hil.held() + awi.held() + awl.held() + live.n + sizeof(int) * gptr.n + sizeof(float2) * cscratch.n +
+               sizeof(float) * (pen.n + ramp.n + scratch.n + qw.n + warp.n + ttau.n) + sizeof(unsigned short) * path.n +
+               sizeof(double) * (nrm.n + gmax.n + dsn.n + dob.n + band.n + vnrm.n + ttm.n);
+    }
 
     // Misfit and adjoint source of every trace (rows of nt samples) of ngather
     // contiguous gathers, all pointers on the device except h_gather_ptr.

@@ -6,6 +6,7 @@
 #include "adjsrc.cuh"
 #include "engine.cuh"
 #include "vmesh.hpp"
+#include "workspace.cuh"
 
 struct owl_ssg {
     std::unique_ptr<owl::Engine> eng;
@@ -328,13 +329,8 @@ int owl_search_direction(int method, long long n, int nm, const float* const* mo
         for (int i = 0; i < nm; ++i) OWL_CHECK(grads[i] && (models[i] || method != OWL_SEARCH_LBFGS),
                                                  OWL_ERR_INVALID, "null model / gradient");
         if (n == 0) return;
-        struct Ctx {
-            cudaStream_t s = nullptr;
-            ~Ctx() {
-                if (s) cudaStreamDestroy(s);
-            }
-        } c;
-        OWL_CUDA(cudaStreamCreateWithFlags(&c.s, cudaStreamNonBlocking));
+        WorkspaceLease ws;
+        Workspace& c = *ws;
         std::vector<const float*> x(nm), g(nm);
         const float* ps = prev_srch;
         float* out = srch;
@@ -355,10 +351,11 @@ int owl_search_direction(int method, long long n, int nm, const float* const* mo
             dsrch.reserve((size_t)n);
             out = dsrch.p;
         }
-        search_direction(method, n, nm, x.data(), g.data(), ps, out, c.s);
+        search_direction(method, n, nm, x.data(), g.data(), ps, out, c);
         if (mem_kind == OWL_MEM_HOST)
             OWL_CUDA(cudaMemcpyAsync(srch, out, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, c.s));
         OWL_CUDA(cudaStreamSynchronize(c.s));
+        ws.done();
     });
 }
 
@@ -370,13 +367,8 @@ int owl_grad_process(int op, int n1, int n2, int n3, const float* param, const f
         OWL_CHECK(n1 >= 1 && n2 >= 1 && n3 >= 1 && field, OWL_ERR_INVALID, "bad field");
         OWL_CHECK(param || op == OWL_GRAD_MASK || op == OWL_GRAD_MAX_BALANCE, OWL_ERR_INVALID, "null param");
         OWL_CHECK(mem_kind == OWL_MEM_HOST || mem_kind == OWL_MEM_DEVICE, OWL_ERR_INVALID, "bad mem_kind");
-        struct Ctx {
-            cudaStream_t s = nullptr;
-            ~Ctx() {
-                if (s) cudaStreamDestroy(s);
-            }
-        } c;
-        OWL_CUDA(cudaStreamCreateWithFlags(&c.s, cudaStreamNonBlocking));
+        WorkspaceLease ws;
+        Workspace& c = *ws;
         const size_t n = (size_t)n1 * n2 * n3;
         DevBuf<float> df, dm;
         float* f = field;
@@ -389,9 +381,10 @@ int owl_grad_process(int op, int n1, int n2, int n3, const float* param, const f
                 m = dm.p;
             }
         }
-        grad_process(op, n1, n2, n3, param, m, f, c.s);
+        grad_process(op, n1, n2, n3, param, m, f, c);
         if (mem_kind == OWL_MEM_HOST) OWL_CUDA(cudaMemcpyAsync(field, f, n * sizeof(float), cudaMemcpyDeviceToHost, c.s));
         OWL_CUDA(cudaStreamSynchronize(c.s));
+        ws.done();
     });
 }
 
@@ -407,14 +400,9 @@ static int adjoint_source_impl(const owl_misfit_opts* mopts, int ngather, const 
         OWL_CHECK(mem_kind == OWL_MEM_HOST || mem_kind == OWL_MEM_DEVICE, OWL_ERR_INVALID, "bad mem_kind");
         const int ntr = ngather ? gather_ptr[ngather] : 0;
         OWL_CHECK(ntr >= 0 && (ntr == 0 || (syn && obs)), OWL_ERR_INVALID, "null trace buffer");
-        struct Ctx {
-            cudaStream_t s = nullptr;
-            ~Ctx() {
-                if (s) cudaStreamDestroy(s);
-            }
-        } c;
-        OWL_CUDA(cudaStreamCreateWithFlags(&c.s, cudaStreamNonBlocking));
-        AdjointSource as;
+        WorkspaceLease ws;
+        Workspace& c = *ws;
+        AdjointSource& as = c.adj;
         const size_t n = (size_t)ntr * nt;
         DevBuf<float> dsyn, dobs, dadj, dw, dtau;
         DevBuf<double> dtm, dgm;
@@ -454,6 +442,7 @@ static int adjoint_source_impl(const owl_misfit_opts* mopts, int ngather, const 
                 OWL_CUDA(cudaMemcpyAsync(gather_misfit, pgm, ngather * sizeof(double), cudaMemcpyDeviceToHost, c.s));
         }
         OWL_CUDA(cudaStreamSynchronize(c.s));
+        ws.done();
     });
 }
 

@@ -97,6 +97,9 @@ void launch_pdl(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStr
     launch_pdl_cluster(k, grid, block, dim3(1, 1, 1), smem, s, args...);
 }
 
+// frees the idle workspaces of the current device (workspace.cu)
+void workspace_trim();
+
 // ----------------------------------------------------------------------------
 // grow-only device buffer. Keeping the pointer stable across calls lets the
 // captured CUDA graphs be replayed without re-instantiation.
@@ -119,7 +122,12 @@ struct DevBuf {
         if (count <= n && p) return false;
         release();
         size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
-        const cudaError_t e = cudaMalloc(&p, bytes);
+        cudaError_t e = cudaMalloc(&p, bytes);
+        if (e == cudaErrorMemoryAllocation) {
+            (void)cudaGetLastError();
+            workspace_trim();
+            e = cudaMalloc(&p, bytes);
+        }
         if (e != cudaSuccess) {
             // a failed allocation leaves the handle usable: clear the runtime's
             // last error so that the next launch check does not report it again

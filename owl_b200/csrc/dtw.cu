@@ -794,10 +794,9 @@ void AdjointSource::run_dtw(const owl_misfit_opts& o, int ngather, int nt, int n
     dob.reserve(nn);
     qw.reserve(nn);
     warp.reserve((size_t)ntr * std::max(nt, ns));
-    DevBuf<float> tmp_tau;
     if (!tau_out) {
-        tmp_tau.reserve(nn);
-        tau_out = tmp_tau.p;
+        ttau.reserve(nn);
+        tau_out = ttau.p;
     }
     a.dsn = dsn.p;
     a.dob = dob.p;

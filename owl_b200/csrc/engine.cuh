@@ -95,9 +95,10 @@ void su_encode(const unsigned char* header, const float* traces, int ntr, int ns
                cudaStream_t s);
 void su_decode(const unsigned char* in, int ntr, int ns, float* traces, bool dev, cudaStream_t s);
 // search directions / gradient processing (optim.cu), device pointers
+struct Workspace;
 void search_direction(int method, long long n, int nm, const float* const* x, const float* const* g,
-                      const float* prev_srch, float* srch, cudaStream_t s);
-void grad_process(int op, int n1, int n2, int n3, const float* param, const float* mask, float* f, cudaStream_t s);
+                      const float* prev_srch, float* srch, Workspace& ws);
+void grad_process(int op, int n1, int n2, int n3, const float* param, const float* mask, float* f, Workspace& ws);
 // out[i] = (w[i] != 0) (adjsrc.cu)
 void launch_nonzero(const float* w, int n, unsigned char* out, cudaStream_t s);
 

