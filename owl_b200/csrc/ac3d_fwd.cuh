@@ -7,6 +7,12 @@
 // is brought into a NS-stage shared-memory ring by 16-byte cp.async copies
 // issued NS-1 planes ahead, so HBM loads overlap the arithmetic without holding
 // registers. z neighbours come from a register queue of 2R values per row.
+// One barrier per plane: a stage is refilled right after the barrier that
+// follows its last reads. Bound by HBM and L2 (halo rows); on B200 the p / v
+// kernels take 486 / 665 us on 440^3 padded cells (497 / 669 us with a second
+// barrier) and 143 / 174 us on 281 x 261 x 241 (146 / 174 us). Reading the CPML
+// memories a plane ahead cost registers (48 -> 64): 614 / 703 us on 440^3, though
+// 49 / 56 instead of 54 / 63 us on 171 x 161 x 151; not used.
 #pragma once
 // (no namespace block: ac3d.cu includes this inside namespace owl)
 
@@ -82,10 +88,11 @@ __global__ void __launch_bounds__(256) k_ac3d_fwd_p(Ac3dDev a) {
             cp_commit();
         }
         for (int z = zb, i = 0; z < ze; ++z, ++i) {
+            cp_wait<AC3_NS - 2>();
+            __syncthreads();
+            // refill the stage that every thread has left behind at this barrier
             if (z + AC3_NS - 1 < ze) issue(z + AC3_NS - 1, (i + AC3_NS - 1) % AC3_NS);
             cp_commit();
-            cp_wait<AC3_NS - 1>();
-            __syncthreads();
             const float* st = ring + (i % AC3_NS) * T::STAGE;
             const int zo = z * pl;
             const bool pz = (!a.fsurf && z < a.pr) || z >= a.pr + a.nz;
@@ -127,7 +134,6 @@ __global__ void __launch_bounds__(256) k_ac3d_fwd_p(Ac3dDev a) {
                 for (int j = 0; j < 2 * R - 1; ++j) q[r][j] = q[r][j + 1];
                 q[r][2 * R - 1] = st[T::OZ + lr * 32 + tx];
             }
-            __syncthreads();
         }
         cp_wait<0>();
         __syncthreads();
@@ -196,10 +202,11 @@ __global__ void __launch_bounds__(256) k_ac3d_fwd_v(Ac3dDev a) {
             cp_commit();
         }
         for (int z = zb, i = 0; z < ze; ++z, ++i) {
+            cp_wait<AC3_NS - 2>();
+            __syncthreads();
+            // refill the stage that every thread has left behind at this barrier
             if (z + AC3_NS - 1 < ze) issue(z + AC3_NS - 1, (i + AC3_NS - 1) % AC3_NS);
             cp_commit();
-            cp_wait<AC3_NS - 1>();
-            __syncthreads();
             const float* st = ring + (i % AC3_NS) * T::STAGE;
             const int zo = z * pl;
             const bool dox = z >= a.zvx0, doz = z >= a.zvz0;
@@ -249,7 +256,6 @@ __global__ void __launch_bounds__(256) k_ac3d_fwd_v(Ac3dDev a) {
                 for (int j = 0; j < 2 * R - 1; ++j) q[r][j] = q[r][j + 1];
                 q[r][2 * R - 1] = st[T::OQ + lr * 32 + tx];
             }
-            __syncthreads();
         }
         cp_wait<0>();
         __syncthreads();
