@@ -1080,9 +1080,10 @@ struct Ac2dEngine : SsgBase {
     }
     // forward steps of the batch run resident: the automatic mode, explosion
     // sources only (force taps enter between the velocity update and the halo
-    // exchange), traces that the threads of one CTA can hold
+    // exchange) whose taps lie inside the updated nodes (the arrays end there),
+    // traces that the threads of one CTA can hold
     bool resident(int pass, int S) override {
-        if (pass != 0 || !res_allowed || fuse_fwd || (inj_fmask & 6)) return false;
+        if (pass != 0 || !res_allowed || fuse_fwd || !taps_inside || (inj_fmask & 6)) return false;
         const ResPlan& p = R == 4 ? res_plan<4>(S) : res_plan<8>(S);
         return p.ok && max_traces <= 2 * p.threads;
     }

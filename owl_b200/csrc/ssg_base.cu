@@ -502,6 +502,7 @@ void SsgBase::build_tables(int S, const owl_shot* shots, bool need_sct) {
     // the separate point kernel, whose one small launch per step costs less
     // than the extra work of the stencil CTAs), OWL_FUSE=0 neither
     const char* fz = std::getenv("OWL_FUSE");
+    taps_inside = fuse;
     fuse_on = fuse && !(fz && fz[0] == '0' && fz[1] == 0);
     fuse_fwd = fuse_on && fz && fz[0] == '1' && fz[1] == 0;
 }

@@ -109,6 +109,7 @@ struct SsgBase : Engine {
     bool want_src_now = false;  // the adjoint sweep records the source-side adjoint
     int fz_mode = 0;       // FZ_* work of the next stencil launches
     bool res_allowed = false;  // this call may run whole segments as one launch (automatic tiles, graphs on)
+    bool taps_inside = false;  // every source tap of the batch lies on a node its kernel updates
     int max_traces = 0;        // most traces of a shot of the batch
     DevBuf<int> inj_last;      // per shot: last step (1-based) whose source amplitudes are not all zero
     DevBuf<unsigned char> live;

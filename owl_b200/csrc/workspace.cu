@@ -40,7 +40,7 @@ unsigned long long context_id() {
 WorkspaceLease::WorkspaceLease() {
     int dev = 0;
     OWL_CUDA(cudaGetDevice(&dev));
-    OWL_CUDA(cudaFree(nullptr));  // the device's context exists from here on
+    OWL_CUDA(cudaSetDevice(dev));  // the device's context exists and is this thread's from here on
     const unsigned long long ctx = context_id();
     {
         std::lock_guard<std::mutex> g(ws_lock());

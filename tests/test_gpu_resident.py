@@ -85,6 +85,13 @@ def test_what_stays_step_by_step():
         a = s.forward(ps, RunOpts())
         assert s.last_info.gpu_launches > 2 * nt
         np.testing.assert_array_equal(a, s.forward(ps, STEPWISE))
+    # taps beyond the absorbing layer of a narrow one, where no node is updated
+    narrow = SSGSolver(L.OWL_ACOUSTIC_ISO_2D, nx, nz, 10.0, 10.0, 1e-3, nt, pml=2, f0_max=12.0)
+    narrow.set_model(vp, rho)
+    ps = narrow.prepare([Shot(1, [Source(x=1.3, z=2.7, f0=12.0)], [Receiver(x=2.0 + 9.0 * i, z=4.0) for i in range(20)])])
+    a = narrow.forward(ps, RunOpts())
+    assert narrow.last_info.gpu_launches > 2 * nt
+    np.testing.assert_array_equal(a, narrow.forward(ps, STEPWISE))
     ps = s.prepare(shots_of(2, nx, nz, False))
     a = s.forward(ps, RunOpts())
     assert s.last_info.gpu_launches < nt
