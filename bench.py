@@ -611,6 +611,13 @@ def headline_roofline(s, d, k, peak, peak_kind):
     # the other segments storing; adjoint every step
     counts = {L.OWL_K_FWD_P: nt - n_last, L.OWL_K_FWD_V: nt - n_last, L.OWL_K_FWD_P_STORE: nt,
               L.OWL_K_FWD_V_STORE: nt, L.OWL_K_ADJ_P: nt, L.OWL_K_ADJ_V: nt}
+    # the forward and recomputed segments run as one launch each with the state in
+    # shared memory (no step kernels) where a gradient has about two launches per
+    # step: the adjoint's
+    resident = s.last_info.gpu_launches < 3 * nt
+    if resident:
+        for kid in (L.OWL_K_FWD_P, L.OWL_K_FWD_V, L.OWL_K_FWD_P_STORE, L.OWL_K_FWD_V_STORE):
+            counts[kid] = 0
     # the autotuner's variants: tile codes 100 + h are the four-cell kernels,
     # 200 + h the same with the pipelined adjoint p kernel, 300 + h the
     # one-cell kernels with it (pipelined only when a CTA takes several shots)
@@ -637,6 +644,7 @@ def headline_roofline(s, d, k, peak, peak_kind):
             "frac": achieved / peak, "peak_source": peak_kind, "traffic": profile_traffic(short),
             "alg_bytes_per_launch": bytes_k, "ms_per_launch": ms_k,
             "kernel_ms_per_launch": {names[q]: kt[q][0] for q in kt},
+            "forward": "k_ac2d_fwd_res: one launch per segment, state in shared memory" if resident else "step kernels",
             "launches_per_gradient": {names[q]: counts[q] for q in kt},
             "kernel_ms_per_gradient": {names[q]: kt[q][0] * counts[q] for q in kt},
             "tile_codes": {"forward": s.last_info.tile_z_forward, "adjoint": s.last_info.tile_z,
@@ -772,8 +780,10 @@ def main():
         "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic",
         "config": workload_config(world, nshots),
         "algorithm": "exact discrete adjoint, FP32 checkpoints every 50 steps with segment recompute (the "
-                     "forward stores the last segment's stencil terms), all shots of a GPU in each stencil "
-                     "launch, CUDA-graph time loop; FP64 misfit, chain rule and cross-rank reductions",
+                     "forward stores the last segment's stencil terms); forward and recomputed segments with "
+                     "the state resident in shared memory (one cluster per shot), the adjoint with all shots of "
+                     "a GPU in each stencil launch, CUDA-graph time loop; FP64 misfit, chain rule and cross-rank "
+                     "reductions",
         "gcells_per_s": gcells,
         "wall_s_timed": wall,
         "e2e": {"value": e2e_value, "unit": "s/shot", "h2d_bytes_per_step": int(obs.nbytes),
