@@ -74,8 +74,14 @@ def test_resident_segments_equal_step_launches(nx, nz, pml, half, fs, nshots, nt
         assert np.linalg.norm(h0 - h1) <= 2e-6 * np.linalg.norm(h1)
 
 
+def close(a, b):
+    """The automatic step kernels may be the four-cell ones, which round a few sums differently."""
+    assert np.linalg.norm(a - b) <= 2e-6 * np.linalg.norm(b)
+
+
 def test_what_stays_step_by_step():
-    """Force sources, more traces than a CTA's threads hold, explicit tiles and plain launches."""
+    """Force sources, more traces than a CTA's threads hold, taps beyond the updated nodes, explicit tiles and
+    plain launches."""
     nx, nz, nt = 64, 48, 60
     vp, rho = model(nz, nx)
     s = SSGSolver(L.OWL_ACOUSTIC_ISO_2D, nx, nz, 10.0, 10.0, 1e-3, nt, pml=10, f0_max=12.0, max_shots=2)
@@ -84,14 +90,14 @@ def test_what_stays_step_by_step():
         ps = s.prepare(shots)
         a = s.forward(ps, RunOpts())
         assert s.last_info.gpu_launches > 2 * nt
-        np.testing.assert_array_equal(a, s.forward(ps, STEPWISE))
+        close(a, s.forward(ps, STEPWISE))
     # taps beyond the absorbing layer of a narrow one, where no node is updated
     narrow = SSGSolver(L.OWL_ACOUSTIC_ISO_2D, nx, nz, 10.0, 10.0, 1e-3, nt, pml=2, f0_max=12.0)
     narrow.set_model(vp, rho)
     ps = narrow.prepare([Shot(1, [Source(x=1.3, z=2.7, f0=12.0)], [Receiver(x=2.0 + 9.0 * i, z=4.0) for i in range(20)])])
     a = narrow.forward(ps, RunOpts())
     assert narrow.last_info.gpu_launches > 2 * nt
-    np.testing.assert_array_equal(a, narrow.forward(ps, STEPWISE))
+    close(a, narrow.forward(ps, STEPWISE))
     ps = s.prepare(shots_of(2, nx, nz, False))
     a = s.forward(ps, RunOpts())
     assert s.last_info.gpu_launches < nt
