@@ -19,17 +19,11 @@
 #include <cmath>
 
 #include "adjsrc.cuh"
+#include "dtw_row.cuh"
 
 namespace owl {
 
 namespace {
-
-constexpr double DTW_SMIN = 1.0e-8, DTW_SMAX = 1.0e2, DTW_ETA = 0.15, DTW_DELTA = 1.0e-10;
-constexpr double DTW_HUGE = 1.7976931348623157e308;
-
-__device__ __forceinline__ double dadd(double a, double b) { return __dadd_rn(a, b); }
-__device__ __forceinline__ double dsub(double a, double b) { return __dsub_rn(a, b); }
-__device__ __forceinline__ double dmul(double a, double b) { return __dmul_rn(a, b); }
 
 struct DtwArgs {
     int n, m, ntr, ngather, niter, trc, form;
@@ -129,22 +123,6 @@ __global__ void k_dtw_normalise(DtwArgs a) {
     }
 }
 
-// x / b, correctly rounded, for a divisor b used many times, with its reciprocal
-// as rh + rl (rh = RN(1 / b), rl the rounded remainder): x rh + x rl lies within
-// half an ulp and a little of the quotient, its remainder is exact in one
-// multiply-add, and the last multiply-add rounds correctly (Markstein,
-// Computation of elementary functions on the IBM RISC System/6000 processor,
-// IBM J. Res. Dev. 34, 1990). For finite x whose quotient and remainder stay
-// in the normal range, as the grid positions and slopes here do.
-struct DivBy {
-    double b, rh, rl;
-    __device__ explicit DivBy(double b_) : b(b_), rh(1.0 / b_) { rl = __dmul_rn(__fma_rn(-b, rh, 1.0), rh); }
-};
-__device__ __forceinline__ double ddivby(double x, const DivBy& d) {
-    const double q = __fma_rn(x, d.rh, __dmul_rn(x, d.rl));
-    return __fma_rn(__fma_rn(-d.b, q, x), d.rh, q);
-}
-
 // linear interpolation of column x (uniform grid i / (n-1)) at q, clamped to the ends
 // (g: division by n - 1)
 __device__ __forceinline__ double interp_clamped(const double* x, int n, double q, const DivBy& g) {
@@ -172,9 +150,9 @@ __device__ __forceinline__ double powabs(double d, double p) {
 // The program is a chain of n - 1 dependent rows; a row is m candidates times
 // the run of predecessors whose slope is allowed (all j <= k once the band has
 // shrunk). A group of G lanes takes one candidate and strides over its
-// predecessors twice: first the costs in single precision, whose least value and
-// error bound leave one or a few predecessors; then those alone in the
-// program's double arithmetic (least cost, ties to the lowest predecessor, as
+// predecessors twice (dtw_row.cuh): first the costs in single precision, whose
+// least value and error bound leave one or a few predecessors; then those alone in
+// the program's double arithmetic (least cost, ties to the lowest predecessor, as
 // the reference's ascending strict comparison). What depends on the band alone
 // (grid positions, node costs with their interpolation, square root and
 // divisions) is computed for DTW_ROWS rows at once by all threads, ahead of the
@@ -204,8 +182,7 @@ __global__ void __launch_bounds__(DTW_THREADS, 2) k_dtw_solve(DtwArgs a, int lg,
     unsigned short* anc_a = reinterpret_cast<unsigned short*>(f32b + m);
     unsigned short* anc_b = anc_a + m;
     __shared__ double s_cost;
-    __shared__ float2 scs[DTW_ROWS];  // candidates per unit of position (0: a band too narrow to locate
-                                      // candidates in) and the slope's change per candidate
+    __shared__ DtwScale scs[DTW_ROWS];
     __shared__ unsigned short jb[16384 / DTW_TRACE + 2];  // path's candidate at each multiple of DTW_TRACE rows
     const int nblk = (n - 1) / DTW_TRACE;
     unsigned short* path = a.path + (size_t)blockIdx.x * (n + nblk + 1) * m;
@@ -213,21 +190,8 @@ __global__ void __launch_bounds__(DTW_THREADS, 2) k_dtw_solve(DtwArgs a, int lg,
     double* L = a.band + (size_t)blockIdx.x * 3 * n;
     double* U = L + n;
     double* T = U + n;
-    const double dt = 1.0 / ((double)n - 1.0);
-    const DivBy gdt(dt), gn((double)(n - 1));
-    // slope s = RN(x / dt) of a step x allowed (s_min - delta <= s <= s_max + delta) exactly
-    // for x_min <= x <= x_max
-    // (the products are off by an ulp at most; the searches are bounded all the same)
-    double x_max = dmul(DTW_SMAX + DTW_DELTA, dt), x_min = dmul(DTW_SMIN - DTW_DELTA, dt);
-    auto above = [&](double x) { return ddivby(x, gdt) > DTW_SMAX + DTW_DELTA; };
-    auto below = [&](double x) { return ddivby(x, gdt) < DTW_SMIN - DTW_DELTA; };
-    for (int i = 0; i < 8 && above(x_max); ++i) x_max = nextafter(x_max, 0.0);
-    for (int i = 0; i < 8 && !above(nextafter(x_max, DTW_HUGE)); ++i) x_max = nextafter(x_max, DTW_HUGE);
-    for (int i = 0; i < 8 && below(x_min); ++i) x_min = nextafter(x_min, DTW_HUGE);
-    for (int i = 0; i < 8 && !below(nextafter(x_min, 0.0)); ++i) x_min = nextafter(x_min, 0.0);
-    const float rdt = (float)(1.0 / dt), cr = (float)dmul(dt, a.rinst);
-    constexpr float EPS = 5.9604645e-8f;  // 2^-24
-    const float dpos = 1.0e-15f * rdt;    // slope error of rounded positions
+    const DtwSlopes w(n, a.rinst);
+    const DivBy gn((double)(n - 1));
     const int G = 1 << lg, glane = threadIdx.x & (G - 1), kbase = threadIdx.x >> lg, ngrp = blockDim.x >> lg;
     for (int j = threadIdx.x; j < m; j += blockDim.x) lin[j] = (double)j / (double)(m - 1);
     for (int r = blockIdx.x; r < a.ntr; r += gridDim.x) {
@@ -309,87 +273,30 @@ __global__ void __launch_bounds__(DTW_THREADS, 2) k_dtw_solve(DtwArgs a, int lg,
                 }
                 if ((int)threadIdx.x < nrow) {
                     const int i = i0 + threadIdx.x;
-                    const double du = dsub(U[i], L[i]);
-                    const double sc = du > 1.0e-9 ? (double)(m - 1) / du : 0.0;
-                    scs[threadIdx.x] = make_float2((float)sc, sc > 0.0 ? (float)(1.0 / (sc * dt)) : 0.f);
+                    scs[threadIdx.x] = dtw_scale(dsub(U[i], L[i]), m, w.dt);
                 }
                 __syncthreads();
                 for (int rr = 0; rr < nrow; ++rr) {
                     const int row = i0 + rr + 1;
                     const double* tc = taus + rr * m;
-                    const double li = tc[0];
-                    const float sc = scs[rr].x, c1 = scs[rr].y;
+                    const DtwScale sc = scs[rr];
                     // (whole warps go round together: a shuffle of each group by itself would run the
                     // groups of a warp one after the other)
                     for (int k0 = kbase; k0 - kbase < m; k0 += ngrp) {
                         const int k = min(k0, m - 1);
                         const double tgk = tc[m + k];
                         const double nu = nus[rr * m + k];
-                        double best = DTW_HUGE;
-                        int bj = 0;
-                        auto exact = [&](int j) {  // (an unreachable predecessor, DTW_HUGE, never gives a lower cost)
-                            const double sl = ddivby(dsub(tgk, tc[j]), gdt);
-                            const double pc = dadd(fcur[j], dmul(dt, dadd(dmul(a.rinst, dmul(sl, sl)), nu)));
-                            if (pc < best || (pc == best && j < bj)) {
-                                best = pc;
-                                bj = j;
-                            }
-                        };
-                        auto allowed = [&](int j) {
-                            const double x = dsub(tgk, tc[j]);
-                            return x <= x_max && x >= x_min;
-                        };
-                        if (sc > 0.f) {
-                            // candidates of an allowed slope form one run (the slope falls as j grows): a
-                            // window [jlo, jhi] that holds it, two candidates to spare (the estimate is off
-                            // by less than one); all but its outer five at each end are allowed for certain
-                            const float e0 = (float)(tgk - x_max - li) * sc, e1 = (float)(tgk - x_min - li) * sc;
-                            const int jlo = e0 <= 2.f ? 0 : (int)fminf(e0, (float)m) - 2;
-                            const int jhi = e1 >= (float)(m - 3) ? m - 1 : (int)fmaxf(e1, -3.f) + 2;
-                            const int in0 = jlo + 5, in1 = jhi - 5;
-                            const int na = in1 < in0 ? jhi - jlo + 1 : 5, ne = in1 < in0 ? na : 10;
-                            // costs without the node's own term, in single precision: s falls by c1 per
-                            // candidate from its value at jlo
-                            const float s0 = (float)dsub(tgk, tc[min(jlo, m - 1)]) * rdt;
-                            auto cost32 = [&](int j) {
-                                const float sl = fmaf(-c1, (float)(j - jlo), s0);
-                                return fmaf(sl * sl, cr, gcur[j]);
-                            };
-                            // the lane's least cost, its predecessor, and the second least
-                            float g1 = INFINITY, g2 = INFINITY;
-                            int j1 = 0;
-                            auto take = [&](int j, float v) {
-                                g2 = fminf(g2, fmaxf(g1, v));
-                                if (v < g1) {
-                                    g1 = v;
-                                    j1 = j;
-                                }
-                            };
-#pragma unroll 8
-                            for (int j = in0 + glane; j <= in1; j += G) take(j, cost32(j));
-                            for (int e = glane; e < ne; e += G) {
-                                const int j = e < na ? jlo + e : in1 + 1 + e - na;
-                                if (allowed(j)) take(j, cost32(j));
-                            }
-                            float g = g1;
+                        DtwLane p(w, tc, fcur, gcur, m, glane, G, tgk, nu, sc);
+                        if (sc.sc > 0.f) {
+                            p.screen();
+                            float g = p.g1;
                             for (int o = G / 2; o; o >>= 1) g = fminf(g, __shfl_xor_sync(0xffffffffu, g, o));
-                            // bound of twice the error of a cost: 2 eps of the cost (its predecessor's part
-                            // and the sum) and 10 eps of the largest slope term (s to 3 eps of s0, its square,
-                            // the product), doubled; the positions' own double rounding in the slope, and
-                            // costs too small for single precision
-                            const float sm = fabsf(s0) + c1;
-                            const float thr = g + EPS * (8.f * g + 40.f * (cr * (sm * sm))) +
-                                              4.f * cr * (2.f * sm * dpos + dpos * dpos) + 1.0e-37f;
-                            if (g1 <= thr && g1 < INFINITY) {
-                                exact(j1);
-                                if (g2 <= thr)  // more than one of the lane's within the bound: all of them
-                                    for (int j = jlo + glane; j <= jhi; j += G)
-                                        if (cost32(j) <= thr && allowed(j)) exact(j);
-                            }
+                            p.resolve(g);
                         } else {
-                            for (int j = glane; j < m; j += G)
-                                if (allowed(j)) exact(j);
+                            p.all();
                         }
+                        double best = p.best;
+                        int bj = p.bj;
                         for (int o = G / 2; o; o >>= 1) {
                             const double ob = __shfl_xor_sync(0xffffffffu, best, o);
                             const int oj = __shfl_xor_sync(0xffffffffu, bj, o);
