@@ -155,12 +155,15 @@ struct DtwLane {
     // g: the least g1 over the lanes. The bound is twice the error of a cost: 2 eps of
     // the cost (its predecessor's part and the sum) and 10 eps of the largest slope
     // term (s to 3 eps of s0, its square, the product), doubled; the positions' own
-    // double rounding in the slope; and costs too small for single precision.
+    // double rounding in the slope; costs too small for single precision; and the
+    // double rounding of the program's own cost, the node's term included (five
+    // roundings of 2^-53, twice: where the costs before are far below that term they
+    // tie, and the lowest predecessor wins).
     DTW_HD void resolve(float g) {
         constexpr float EPS = 5.9604645e-8f;  // 2^-24
         const float sm = fabsf(s0) + s.c1;
         const float thr = g + EPS * (8.f * g + 40.f * (w.cr * (sm * sm))) +
-                          4.f * w.cr * (2.f * sm * w.dpos + w.dpos * w.dpos) + 1.0e-37f;
+                          4.f * w.cr * (2.f * sm * w.dpos + w.dpos * w.dpos) + 2.0e-15f * (float)dmul(w.dt, nu) + 1.0e-37f;
         if (g1 <= thr && g1 < INFINITY) {
             exact(j1);
             if (g2 <= thr)  // more than one of the lane's

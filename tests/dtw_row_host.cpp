@@ -146,6 +146,7 @@ int main(int argc, char** argv) {
         {101, 101, 5, 0.1f, 1.0, 0.5, 1.0, 0, false},    // the defaults
         {61, 31, 5, 0.1f, 1.0, 0.5, 1.0, 20, false},     // muted samples
         {61, 31, 5, 0.1f, 1.0, 0.5, 1.0, 0, true},       // equal traces: no distance on the diagonal
+        {47, 65, 20, 0.0, 1.0, 0.5, 1.0, 16, false},     // no slope cost, bands down to rounding
         {47, 33, 12, 0.1f, 0.0, 2.0, 1.0, 16, false},    // no position cost
         {47, 33, 4, 1e30, 1e30, 0.5, 1.0, 8, false},     // costs near the end of single precision
         {47, 33, 4, 1e-38, 1e-38, 2.0, 1e-20, 8, false}, // costs below its normal range
