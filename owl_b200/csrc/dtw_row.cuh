@@ -164,7 +164,9 @@ struct DtwLane {
         const float sm = fabsf(s0) + s.c1;
         const float thr = g + EPS * (8.f * g + 40.f * (w.cr * (sm * sm))) +
                           4.f * w.cr * (2.f * sm * w.dpos + w.dpos * w.dpos) + 2.0e-15f * (float)dmul(w.dt, nu) + 1.0e-37f;
-        if (g1 <= thr && g1 < INFINITY) {
+        if (!(thr < INFINITY)) {  // costs beyond single precision, none reachable, not a number
+            each<1>([&](int j) { exact(j); });
+        } else if (g1 <= thr) {
             exact(j1);
             if (g2 <= thr)  // more than one of the lane's
                 each<1>([&](int j) {

@@ -149,6 +149,8 @@ int main(int argc, char** argv) {
         {47, 65, 20, 0.0, 1.0, 0.5, 1.0, 16, false},     // no slope cost, bands down to rounding
         {47, 33, 12, 0.1f, 0.0, 2.0, 1.0, 16, false},    // no position cost
         {47, 33, 4, 1e30, 1e30, 0.5, 1.0, 8, false},     // costs near the end of single precision
+        {47, 33, 4, 3e38, 3e38, 1.0, 1.0, 8, false},     // and beyond
+        {47, 33, 4, 0.1f, 1.0, 200.0, 3e2, 8, false},    // distances beyond single precision
         {47, 33, 4, 1e-38, 1e-38, 2.0, 1e-20, 8, false}, // costs below its normal range
         {9, 301, 5, 0.1f, 1.0, 0.5, 1.0, 0, false},      // many candidates, few rows
         {400, 5, 5, 0.1f, 1.0, 1.0, 1.0, 0, false},      // few candidates, many rows
