@@ -168,12 +168,12 @@ __device__ __forceinline__ double powabs(double d, double p) {
 constexpr int DTW_THREADS = 512;
 constexpr int DTW_ROWS = 8;    // rows whose node costs are computed at once (fewer where m is large)
 constexpr int DTW_TRACE = 32;  // rows per block of the traceback
+constexpr int DTW_SMEM = 52 * 4095;  // dynamic shared memory at the most candidates
 
 __global__ void __launch_bounds__(DTW_THREADS, 2) k_dtw_solve(DtwArgs a, int lg, int RB) {
     extern __shared__ double sh[];
     const int n = a.n, m = a.m, jc = (m - 1) / 2;
-    double* lin = sh;
-    double* fa = lin + m;
+    double* fa = sh;
     double* fb = fa + m;
     double* taus = fb + m;           // RB + 1 rows of candidate positions
     double* nus = taus + (RB + 1) * m;  // RB rows of node costs
@@ -191,9 +191,9 @@ __global__ void __launch_bounds__(DTW_THREADS, 2) k_dtw_solve(DtwArgs a, int lg,
     double* U = L + n;
     double* T = U + n;
     const DtwSlopes w(n, a.rinst);
-    const DivBy gn((double)(n - 1));
+    const DivBy gn((double)(n - 1)), gm((double)(m - 1));
+    auto lin = [&](int j) { return ddivby((double)j, gm); };  // place of candidate j in the band
     const int G = 1 << lg, glane = threadIdx.x & (G - 1), kbase = threadIdx.x >> lg, ngrp = blockDim.x >> lg;
-    for (int j = threadIdx.x; j < m; j += blockDim.x) lin[j] = (double)j / (double)(m - 1);
     for (int r = blockIdx.x; r < a.ntr; r += gridDim.x) {
         const int g = gather_of(a, r);
         if (g % a.vc != 0) continue;  // dtw-vector: the receiver is solved from its first component's row
@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(DTW_THREADS, 2) k_dtw_solve(DtwArgs a, int lg,
             __syncthreads();
             // row 0: only the centre candidate (bc_start_stop)
             for (int k = threadIdx.x; k < m; k += blockDim.x) {
-                const double f0 = k == jc ? node_cost(0, dadd(L[0], dmul(dsub(U[0], L[0]), lin[k]))) : DTW_HUGE;
+                const double f0 = k == jc ? node_cost(0, dadd(L[0], dmul(dsub(U[0], L[0]), lin(k)))) : DTW_HUGE;
                 fa[k] = f0;
                 f32a[k] = (float)f0;
                 anc_a[k] = (unsigned short)k;
@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(DTW_THREADS, 2) k_dtw_solve(DtwArgs a, int lg,
                 __syncthreads();
                 for (int e = threadIdx.x; e < (nrow + 1) * m; e += blockDim.x) {
                     const int rr = e / m, j = e - rr * m;
-                    const double tg = dadd(L[i0 + rr], dmul(dsub(U[i0 + rr], L[i0 + rr]), lin[j]));
+                    const double tg = dadd(L[i0 + rr], dmul(dsub(U[i0 + rr], L[i0 + rr]), lin(j)));
                     taus[e] = tg;
                     if (rr > 0) nus[e - m] = node_cost(i0 + rr, tg);
                 }
@@ -342,10 +342,10 @@ __global__ void __launch_bounds__(DTW_THREADS, 2) k_dtw_solve(DtwArgs a, int lg,
                 const int first = b * DTW_TRACE, last = b < nblk ? first + DTW_TRACE : n - 1;
                 int j = b < nblk ? jb[b + 1] : jc;
                 for (int i = last; i > first; --i) {
-                    if (b == nblk || i < last) T[i] = dadd(L[i], dmul(dsub(U[i], L[i]), lin[j]));
+                    if (b == nblk || i < last) T[i] = dadd(L[i], dmul(dsub(U[i], L[i]), lin(j)));
                     j = path[(size_t)i * m + j];
                 }
-                T[first] = dadd(L[first], dmul(dsub(U[first], L[first]), lin[j]));
+                T[first] = dadd(L[first], dmul(dsub(U[first], L[first]), lin(j)));
             }
             __syncthreads();
             const double cost = s_cost;
@@ -754,14 +754,16 @@ void AdjointSource::run_dtw(const owl_misfit_opts& o, int ngather, int nt, int n
         b.q = rq.p;
     }
     // lanes per candidate: the most that give every candidate a group; rows of node
-    // costs at once: as many as two CTAs' shared memory holds, at least one
+    // costs at once: as many as two CTAs' shared memory holds, at least one (52 bytes
+    // a candidate: 208 KB of the CTA's 227 KB at the most candidates)
     int lg = 0;
     while (lg < 5 && (2 << lg) * m <= DTW_THREADS) ++lg;
-    auto smem_of = [&](int rb) { return (size_t)m * ((4 + 2 * rb) * sizeof(double) + 2 * sizeof(float) + 2 * sizeof(unsigned short)); };
+    auto smem_of = [&](int rb) { return (size_t)m * ((3 + 2 * rb) * sizeof(double) + 2 * sizeof(float) + 2 * sizeof(unsigned short)); };
     int RB = DTW_ROWS;
     while (RB > 1 && smem_of(RB) > 100 * 1024) --RB;
     const size_t smem = smem_of(RB);
-    OWL_CUDA(cudaFuncSetAttribute(k_dtw_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // (the same limit in every call: calls of several threads may run side by side)
+    OWL_CUDA(cudaFuncSetAttribute(k_dtw_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, DTW_SMEM));
     k_dtw_solve<<<grid, DTW_THREADS, smem, s>>>(b, lg, RB);
     k_dtw_quality<<<ntr, 256, 0, s>>>(b);
     if (rs) {

@@ -79,3 +79,14 @@ def test_dtw_decisions_of_many_traces(pool, nt, m, own):
         mo.dtw_loss_power, mo.dtw_rcuml, mo.dtw_niter = own["power"], own["rcuml"], own["niter"]
     tau = dtw_time_shifts(mo, [0, ntr], syn, obs)
     np.testing.assert_array_equal(tau, ref)
+
+
+@pytest.mark.parametrize("m", [3857, 4095])
+def test_dtw_most_candidates(m):
+    """up to the documented limit of 4095 candidates"""
+    dt, nt, niter = 1e-3, 9, 2
+    syn, obs = _spread(1, nt, dt, m)
+    tlag = float(np.float32(0.5 * (m - 1) * dt))
+    ref = _oracle_shifts((syn, obs, dict(dt=dt, tlag_max=tlag, niter=niter)))
+    tau = dtw_time_shifts(MisfitOpts(misfit=L.OWL_MISFIT_DTW, dt=dt, tlag_max=tlag, dtw_niter=niter), [0, 1], syn, obs)
+    np.testing.assert_array_equal(tau, ref)
