@@ -693,6 +693,14 @@ struct Ac2dEngine : SsgBase {
             for (int irx = -4; irx <= 4; ++irx)
                 taps.push_back(TapPt{0, q.gx + irx, 1, q.gz + irz, q.interp_ix[irx + 4] * q.interp_iz[irz + 4] * q.weight});
     }
+    bool rec_window(const owl_receiver& q, int& i, int& k, float* fx, float* fz, float& w) const override {
+        i = q.gx - 4;
+        k = q.gz - 4;
+        std::copy(q.interp_ix, q.interp_ix + BOX_W, fx);
+        std::copy(q.interp_iz, q.interp_iz + BOX_W, fz);
+        w = q.weight;
+        return true;
+    }
     // with a free surface, p(i, 2-j) = -p(i, j) for j <= 0 and p(i, 1) = 0
     void scatter_map(const TapPt& t, std::vector<TapPt>& out) const override {
         if (!desc.free_surface) { out.push_back(t); return; }
@@ -1095,6 +1103,8 @@ struct Ac2dEngine : SsgBase {
         q.n = n;
         q.smp = kind != 1;
         q.inj_last = inj_last.p;
+        q.org = rec_org.p;
+        q.fac = rec_fac.p;
         const bool store = kind == 1 || kind == 3;
         const ResKernel k = res_kernel<RR>(p.H, store, p.one);
         cudaLaunchConfig_t cfg = {};

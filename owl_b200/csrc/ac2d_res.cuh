@@ -33,7 +33,7 @@
 #pragma once
 
 constexpr int RES_MAXC = 16;     // CTAs of a cluster (above 8: non-portable size)
-constexpr int RES_THREADS = 448;  // 144 registers a thread
+constexpr int RES_THREADS = 448;  // (128 registers a thread)
 constexpr size_t RES_SMEM = 227 * 1024;
 
 struct Ac2dRes {
@@ -45,6 +45,8 @@ struct Ac2dRes {
     int smp;          // record receivers
     int zb[RES_MAXC + 1];  // first resident row of each CTA, relative to zlo
     const int* inj_last;   // per shot: last step (1-based) with a nonzero amplitude
+    const int2* org;       // traces of several taps: storage (x, z) of the window's first tap
+    const float* fac;      // and the factors of its weights, [k][trace]: BOX_W along x, BOX_W along z, the trace's weight
 };
 
 __device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -225,10 +227,9 @@ __device__ float res_read_p(const Ac2dDev& a, const Ac2dRes& q, const ResCta<R>&
 // one trace of the shot at step index cur (0-based): p plus the pending
 // explosion taps, each trace a sequential sum over its taps
 template <int R>
-__device__ __noinline__ float res_sample(const Ac2dDev& a, const Ac2dRes& q, ResCta<R> c, int j0, int j1,
-                                         bool pend, int cur) {
+__device__ __noinline__ float res_sample(const Ac2dDev& a, const Ac2dRes& q, ResCta<R> c, int r, bool pend, int cur) {
     float acc = 0.f;
-    for (int j = j0; j < j1; ++j) {
+    for (int j = a.pt.smp.ptr[r]; j < a.pt.smp.ptr[r + 1]; ++j) {
         const long long off = a.pt.smp.off[j];
         const int z = (int)(off / a.pitch), x = (int)(off - (long long)z * a.pitch);
         float v = res_read_p<R>(a, q, c, z, x);
@@ -238,51 +239,62 @@ __device__ __noinline__ float res_sample(const Ac2dDev& a, const Ac2dRes& q, Res
     return acc;
 }
 
-// the explosion taps of step index ti (0-based) into the CTA's own rows, items
-// it0 and on, in order
+// The shot's injection items, one tap per thread. The first one's tap stays in
+// registers for the launch, its amplitude read a phase ahead; further items are read
+// per step, each while the one before is added.
+struct ResTap {
+    int o;    // shared offset of the thread's tap on the CTA's rows (-1: none)
+    float w;
+};
+struct ResSrc {
+    int last;     // last step (1-based) with a nonzero amplitude
+    int it, nit;
+    bool halo;    // the halo rows take the taps too
+    ResTap t;
+    float A;
+};
 template <int R>
-__device__ __noinline__ void res_inject_items(const Ac2dDev& a, const Ac2dRes& q, ResCta<R> c, int it0, int ti) {
-    const Ac2dPt& t = a.pt;
-    for (int it = it0; it < t.item_ptr[c.s + 1]; ++it) {
-        const int4 b = t.box[it];
-        const float A = t.amp[(size_t)it * t.nt + ti];
-        if (b.x == 0 && A != 0.f) {
-            for (int e = threadIdx.x; e < BOX_W * BOX_W; e += blockDim.x) {
-                const int l = b.w + e / BOX_W - q.zlo - c.l0, x = b.y + e % BOX_W;
-                const float w = t.bw[(size_t)it * (BOX_W * BOX_W) + e];
-                if (l >= 0 && l < c.nr && x >= a.x0 && x < a.x1 && w != 0.f) {
-                    float* f = c.p + (size_t)(l + R) * q.XP + (x - a.x0) + R;
-                    *f = *f + A * w;
-                }
-            }
+__device__ __forceinline__ ResTap res_tap(const Ac2dDev& a, const Ac2dRes& q, const ResCta<R>& c, int it, bool halo) {
+    ResTap t{-1, 0.f};
+    if (threadIdx.x < BOX_W * BOX_W) {
+        const int4 b = __ldg(a.pt.box + it);
+        const int l = b.w + (int)threadIdx.x / BOX_W - q.zlo - c.l0, x = b.y + (int)threadIdx.x % BOX_W;
+        const int h = halo ? R : 0;
+        t.w = __ldg(a.pt.bw + (size_t)it * (BOX_W * BOX_W) + threadIdx.x);
+        if (b.x == 0 && l >= -h && l < c.nr + h && x >= a.x0 && x < a.x1 && t.w != 0.f)
+            t.o = (l + R) * q.XP + (x - a.x0) + R;
+    }
+    return t;
+}
+// items it0 and on of step index ti (0-based), in order
+template <int R>
+__device__ __noinline__ void res_inject_items(const Ac2dDev& a, const Ac2dRes& q, ResCta<R> c, int it0, int ti, bool halo) {
+    const int end = a.pt.item_ptr[c.s + 1], nt = a.pt.nt;
+    const float* amp = a.pt.amp + ti;
+    ResTap t = res_tap<R>(a, q, c, it0, halo);
+    float A = __ldg(amp + (size_t)it0 * nt);
+    for (int it = it0; it < end; ++it) {
+        const ResTap cur = t;
+        const float Ac = A;
+        if (it + 1 < end) {
+            t = res_tap<R>(a, q, c, it + 1, halo);
+            A = __ldg(amp + (size_t)(it + 1) * nt);
         }
+        if (cur.o >= 0 && Ac != 0.f) c.p[cur.o] = c.p[cur.o] + Ac * cur.w;
         __syncthreads();
     }
 }
-
-// The shot's first injection item, one tap per thread held in registers for the
-// launch, its amplitude read a phase ahead; further items are read per step.
-struct ResSrc {
-    int last;   // last step (1-based) with a nonzero amplitude
-    int it, nit;
-    int o;      // the thread's tap on the CTA's rows (-1: none)
-    float w, A;
-};
 template <int R>
-__device__ __forceinline__ void res_find_source(const Ac2dDev& a, const Ac2dRes& q, const ResCta<R>& c, ResSrc& src) {
+__device__ __forceinline__ void res_find_source(const Ac2dDev& a, const Ac2dRes& q, const ResCta<R>& c, bool halo,
+                                                ResSrc& src) {
     const Ac2dPt& t = a.pt;
     src.last = q.inj_last[c.s];
     src.it = t.item_ptr[c.s];
     src.nit = t.item_ptr[c.s + 1] - src.it;
-    src.o = -1;
-    src.w = src.A = 0.f;
-    if (src.nit > 0 && threadIdx.x < BOX_W * BOX_W) {
-        const int4 b = t.box[src.it];
-        const int l = b.w + (int)threadIdx.x / BOX_W - q.zlo - c.l0, x = b.y + (int)threadIdx.x % BOX_W;
-        src.w = t.bw[(size_t)src.it * (BOX_W * BOX_W) + threadIdx.x];
-        if (b.x == 0 && l >= 0 && l < c.nr && x >= a.x0 && x < a.x1 && src.w != 0.f)
-            src.o = (l + R) * q.XP + (x - a.x0) + R;
-    }
+    src.halo = halo;
+    src.t = ResTap{-1, 0.f};
+    src.A = 0.f;
+    if (src.nit > 0) src.t = res_tap<R>(a, q, c, src.it, halo);
 }
 // the taps of step index ti, whose amplitude of the first item is src.A; every
 // thread of the CTA calls it, and the rows are complete after it
@@ -290,20 +302,27 @@ template <int R>
 __device__ __forceinline__ void res_inject(const Ac2dDev& a, const Ac2dRes& q, const ResCta<R>& c, const ResSrc& src,
                                            int ti) {
     if (ti + 1 > src.last) return;
-    if (src.o >= 0 && src.A != 0.f) c.p[src.o] = c.p[src.o] + src.A * src.w;
+    if (src.t.o >= 0 && src.A != 0.f) c.p[src.t.o] = c.p[src.t.o] + src.A * src.t.w;
     __syncthreads();
-    if (src.nit > 1) res_inject_items<R>(a, q, c, src.it + 1, ti);
+    if (src.nit > 1) res_inject_items<R>(a, q, c, src.it + 1, ti, src.halo);
 }
 
-// receivers of the CTA: those whose first tap lies on its rows, up to two per
-// thread, found once per launch (`list`: shared scratch of 1 + 2 blockDim ints)
-enum { RES_NONE = 0, RES_TAP, RES_LOCAL, RES_SPAN };
+// Receivers of the CTA, up to two per thread, found once per launch (`list`:
+// shared scratch of 1 + 2 blockDim ints). A trace of one tap belongs to the CTA of
+// its row, one of several to the CTA of its window's middle row: the window then
+// lies on the CTA's rows and its halo rows, which hold p of the same step from the
+// end of the P phase on.
+enum { RES_NONE = 0, RES_TAP, RES_BOX, RES_NEAR, RES_SPAN };
 struct ResRec {
-    int kind;       // one tap / several taps, all on the CTA's rows; taps of other CTAs or above the surface
-    int r, j0, j1;  // trace, taps
-    int o;          // shared offset of a single tap
-    float w;
+    int kind;  // one tap / a window on the CTA's own and halo rows / one that meets the taps of the shot's sources /
+               // taps beyond the CTA's rows
+    int r;     // trace
+    int o;     // shared offset of the tap, or of the window's first one
+    float w;   // the tap's weight
 };
+// halo rows of p below the CTA's last row that hold p
+template <int R>
+constexpr int RES_BELOW = R < BOX_W / 2 + 1 ? R : R - 1;
 template <int R>
 __device__ __forceinline__ int res_local(const Ac2dDev& a, const Ac2dRes& q, const ResCta<R>& c, long long off) {
     const int z = (int)(off / a.pitch), x = (int)(off - (long long)z * a.pitch), l = z - q.zlo - c.l0;
@@ -315,11 +334,14 @@ __device__ __forceinline__ bool res_find_receivers(const Ac2dDev& a, const Ac2dR
     if (threadIdx.x == 0) list[0] = 0;
     __syncthreads();
     const Ac2dPt& t = a.pt;
+    bool near = false;  // some window of the shot, on whichever CTA, meets the taps of its sources
     if (q.smp)
         for (int r = t.rec_ptr[c.s] + threadIdx.x; r < t.rec_ptr[c.s + 1]; r += blockDim.x) {
-            const int j = t.smp.ptr[r];
-            if (j >= t.smp.ptr[r + 1]) continue;  // no taps: the trace is zero
-            int l = (int)(t.smp.off[j] / a.pitch) - q.zlo;
+            const int j = t.smp.ptr[r], n = t.smp.ptr[r + 1] - j;
+            if (n == 0) continue;  // no taps: the trace is zero
+            const int2 g = n == 1 ? make_int2(0, 0) : q.org[r];
+            near |= n > 1 && ac2d_inj_near(t, c.s, 1, g.x, g.x + BOX_W, g.y, g.y + BOX_W);
+            int l = (n == 1 ? (int)(t.smp.off[j] / a.pitch) : g.y + BOX_W / 2) - q.zlo;
             l = min(max(l, 0), q.zb[q.C] - 1) - c.l0;
             if (l >= 0 && l < c.nr) {
                 const int k = atomicAdd(list, 1);
@@ -334,37 +356,64 @@ __device__ __forceinline__ bool res_find_receivers(const Ac2dDev& a, const Ac2dR
         rec[e].kind = RES_NONE;
         if (k < count) {
             const int r = list[1 + k];
+            const int j = t.smp.ptr[r];
             rec[e].r = r;
-            rec[e].j0 = t.smp.ptr[r];
-            rec[e].j1 = t.smp.ptr[r + 1];
-            rec[e].w = t.smp.w[rec[e].j0];
-            rec[e].o = res_local<R>(a, q, c, t.smp.off[rec[e].j0]);
-            rec[e].kind = rec[e].j1 == rec[e].j0 + 1 ? RES_TAP : RES_LOCAL;
-            for (int j = rec[e].j0; j < rec[e].j1; ++j)
-                if (res_local<R>(a, q, c, t.smp.off[j]) < 0) rec[e].kind = RES_SPAN;
+            if (t.smp.ptr[r + 1] == j + 1) {
+                rec[e].w = t.smp.w[j];
+                rec[e].o = res_local<R>(a, q, c, t.smp.off[j]);
+                rec[e].kind = rec[e].o >= 0 ? RES_TAP : RES_SPAN;
+            } else {
+                const int2 g = q.org[r];
+                const int l = g.y - q.zlo - c.l0, x = g.x - a.x0;
+                rec[e].o = (l + R) * q.XP + x + R;
+                rec[e].kind = l < -R || l + BOX_W > c.nr + RES_BELOW<R> || x < -R || x + BOX_W > 4 * q.XG + R ? RES_SPAN
+                              : ac2d_inj_near(t, c.s, 1, g.x, g.x + BOX_W, g.y, g.y + BOX_W)                  ? RES_NEAR
+                                                                                                              : RES_BOX;
+            }
         }
     }
-    __syncthreads();
-    return count > 0;
+    return __syncthreads_or(near);
 }
-// record the receivers whose taps lie on the CTA's rows, from p with the step's
-// injection, as trace row `row`; complete (for every thread) after it
-template <int R>
-__device__ __noinline__ float res_sample_local(const Ac2dDev& a, const Ac2dRes& q, ResCta<R> c, int j0, int j1) {
+// a trace of several taps from the CTA's own and halo rows: the taps in order (z
+// outer), weight by weight as the tables have them. The window's values lie at
+// fixed offsets, the factors are read coalesced over the traces (19 floats each) and
+// nothing goes through the kernel's parameters. A step of a one-shot 100 x 80 grid
+// takes 2.5 us with traces on nodes, 3.2 us with 20 or 100 such ones and 4.8 us while
+// sources that their windows meet are active; through the taps' own tables, one tap
+// after another with its divisions, it took 61 us (13.8 us step by step).
+__device__ __noinline__ float res_box(const float* __restrict__ f, int n, int XP, int o) {
+    extern __shared__ __align__(16) float res_sm[];
+    float fx[BOX_W], fz[BOX_W];
+#pragma unroll
+    for (int i = 0; i < BOX_W; ++i) {
+        fx[i] = __ldg(f + (size_t)i * n);
+        fz[i] = __ldg(f + (size_t)(BOX_W + i) * n);
+    }
+    const float wt = __ldg(f + (size_t)2 * BOX_W * n);
     float acc = 0.f;
-    for (int j = j0; j < j1; ++j) acc = acc + c.p[res_local<R>(a, q, c, a.pt.smp.off[j])] * a.pt.smp.w[j];
+#pragma unroll
+    for (int k = 0; k < BOX_W; ++k) {
+        float v[BOX_W];
+#pragma unroll
+        for (int i = 0; i < BOX_W; ++i) v[i] = res_sm[o + k * XP + i];
+#pragma unroll
+        for (int i = 0; i < BOX_W; ++i) {
+            const float w = __fmul_rn(__fmul_rn(fx[i], fz[k]), wt);
+            if (w != 0.f) acc = acc + v[i] * w;
+        }
+    }
     return acc;
 }
-template <int R>
-__device__ __forceinline__ void res_record(const Ac2dDev& a, const Ac2dRes& q, const ResCta<R>& c,
-                                           const ResRec (&rec)[2], int row) {
+// record the CTA's traces of one tap, and with `near` those whose windows meet the
+// sources' taps, from p with the step's injection (halo rows included then), as
+// trace row `row`; complete (for every thread) after it
+__device__ __forceinline__ void res_record(const Ac2dDev& a, const Ac2dRes& q, const float* p, const ResRec (&rec)[2],
+                                           int row, bool near) {
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-        if (rec[e].kind != RES_TAP && rec[e].kind != RES_LOCAL) continue;
-        float v;
-        if (rec[e].kind == RES_TAP) v = 0.f + c.p[rec[e].o] * rec[e].w;
-        else v = res_sample_local<R>(a, q, c, rec[e].j0, rec[e].j1);
-        a.pt.rec[(size_t)row * a.pt.rtot + rec[e].r] = v;
+        float* out = a.pt.rec + (size_t)row * a.pt.rtot + rec[e].r;
+        if (rec[e].kind == RES_TAP) *out = 0.f + p[rec[e].o] * rec[e].w;
+        if (near && rec[e].kind == RES_NEAR) *out = res_box(q.fac + rec[e].r, a.pt.rtot, q.XP, rec[e].o);
     }
     __syncthreads();
 }
@@ -498,9 +547,10 @@ __device__ __forceinline__ ResItem<R, H> res_item(const Ac2dDev& a, const Ac2dRe
         if (!(a.fsurf && c.rank == 0 && l == 0)) t.live |= 1u << h;
         if (c.pz_i(l)) t.pi |= 1u << h;
         if (c.pz_h(l)) t.ph |= 1u << h;
-        // p: my rows 0 .. R - 2 follow the CTA above, my last R rows precede the CTA below;
+        // p: my rows 0 .. R - 2 follow the CTA above (at half-width 4 row R - 1 too, for its traces' windows), my
+        // last R rows precede the CTA below;
         // vz: my rows 0 .. R - 1 follow the CTA above, my last R - 1 rows precede the CTA below
-        if (c.rank > 0 && l < R - 1) t.up |= 1u << h;
+        if (c.rank > 0 && l < RES_BELOW<R>) t.up |= 1u << h;
         if (c.rank > 0 && l < R) t.uv |= 1u << h;
         if (c.rank + 1 < q.C && l >= c.nr - R) t.dp |= 1u << h;
         if (c.rank + 1 < q.C && l > c.nr - R) t.dv |= 1u << h;
@@ -717,9 +767,10 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_ac2d_fwd_res(const __grid_co
     res_setup<R>(a, q, res_sm, c);
     const int cur0 = *a.d_step;
     ResRec rec[2];
-    const bool any_rec = res_find_receivers<R>(a, q, c, reinterpret_cast<int*>(res_sm), rec);
+    const bool near = res_find_receivers<R>(a, q, c, reinterpret_cast<int*>(res_sm), rec);
+    const bool taps = __syncthreads_or(rec[0].kind == RES_TAP || rec[1].kind == RES_TAP);
     ResSrc src;
-    res_find_source<R>(a, q, c, src);
+    res_find_source<R>(a, q, c, near, src);
     const float* amp = a.pt.amp + (size_t)src.it * a.pt.nt;
     res_coefs<R>(a, q, c);
     res_load_state<R>(a, q, c);
@@ -743,10 +794,16 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_ac2d_fwd_res(const __grid_co
         const int cur = cur0 + i;
         const long long slot = STORE ? (long long)(cur % a.k) * a.sslot : 0;
         cluster_wait();
-        // explosion sources, then receivers, of the step before
+        // explosion sources, then receivers, of the step before; where windows meet the sources' taps, the taps go
+        // into the halo rows too (each CTA adds the same), which the neighbours' next rows may replace only after that
         if (i > 0) {
+            const bool meet = near && cur <= src.last;
             res_inject<R>(a, q, c, src, cur - 1);
-            if (any_rec) res_record<R>(a, q, c, rec, cur);
+            if (taps || meet) res_record(a, q, c.p, rec, cur, meet);
+            if (meet) {
+                cluster_arrive();
+                cluster_wait();
+            }
         }
         if (ONE) {
             if ((int)threadIdx.x < items) res_p_item<R, H, STORE>(a, q, c, t0, kind, ck, slot, p_up, p_dn);
@@ -759,13 +816,17 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_ac2d_fwd_res(const __grid_co
         cluster_arrive();
         if (cur + 1 <= src.last && src.nit > 0) src.A = __ldg(amp + cur);
         cluster_wait();
-        // receivers with taps of other CTAs, from p and the pending taps of this step
-        if (any_rec && cur + 2 <= a.pt.nt) {
+        // receivers of several taps or of other CTAs' nodes, from p and the pending taps of this step
+        if (cur + 2 <= a.pt.nt) {
+            const bool pend = cur + 1 <= src.last;
 #pragma unroll
-            for (int e = 0; e < 2; ++e)
-                if (rec[e].kind == RES_SPAN)
-                    a.pt.rec[(size_t)(cur + 1) * a.pt.rtot + rec[e].r] =
-                        res_sample<R>(a, q, c, rec[e].j0, rec[e].j1, cur + 1 <= src.last, cur);
+            for (int e = 0; e < 2; ++e) {
+                float* out = a.pt.rec + (size_t)(cur + 1) * a.pt.rtot + rec[e].r;
+                if (rec[e].kind == RES_BOX || (rec[e].kind == RES_NEAR && !pend))
+                    *out = res_box(q.fac + rec[e].r, a.pt.rtot, q.XP, rec[e].o);
+                else if (rec[e].kind == RES_SPAN)
+                    *out = res_sample<R>(a, q, c, rec[e].r, pend, cur);
+            }
         }
         if (ONE) {
             if ((int)threadIdx.x < items) res_v_item<R, H, STORE>(a, q, c, t0, kind, ck, slot, v_up, v_dn);
@@ -781,7 +842,8 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_ac2d_fwd_res(const __grid_co
     if (a.fsurf) res_save_mirror<R>(a, q, c);
     __syncthreads();
     res_inject<R>(a, q, c, src, cur0 + q.n - 1);
-    if (any_rec && cur0 + q.n + 1 <= a.pt.nt) res_record<R>(a, q, c, rec, cur0 + q.n);
+    const bool meet = near && cur0 + q.n <= src.last;
+    if ((taps || meet) && cur0 + q.n + 1 <= a.pt.nt) res_record(a, q, c.p, rec, cur0 + q.n, meet);
     res_save_state<R>(a, q, c);
     tick_last_block(a.d_step, a.pt.d_done, q.n);
 }

@@ -368,6 +368,10 @@ void SsgBase::build_tables(int S, const owl_shot* shots, bool need_sct) {
     item_src.clear(); item_comp.clear(); item_shot.clear(); item_rho_cell.clear(); item_rho.clear();
     const int nt = desc.nt;
     std::vector<TapPt> taps, mapped;
+    std::vector<int2> horg;       // windows of the traces and their factors, FW floats a trace
+    std::vector<float> hfac;
+    constexpr int FW = 2 * BOX_W + 1;
+    bool spread = false;          // some trace has more than one tap
     rtot = 0;
     for (int s = 0; s < S; ++s) {
         const owl_shot& sh = shots[s];
@@ -420,7 +424,16 @@ void SsgBase::build_tables(int S, const owl_shot* shots, bool need_sct) {
                 const owl_receiver& q = sh.rec[r];
                 const int rg = rtot + comp * sh.nrec + r;
                 hlive.push_back(q.weight != 0.f);
+                {
+                    float f[FW] = {};
+                    int wi = 0, wk = 0;
+                    if (rec_window(q, wi, wk, f, f + BOX_W, f[2 * BOX_W])) {
+                        horg.push_back(int2{wi + pr - 1, wk + pr - 1});
+                        hfac.insert(hfac.end(), f, f + FW);
+                    }
+                }
                 if (q.weight != 0.f) {
+                    const int t0 = hsmp.ntaps();
                     taps.clear();
                     rec_taps(q, comp, taps);
                     for (const TapPt& t : taps) {
@@ -438,6 +451,7 @@ void SsgBase::build_tables(int S, const owl_shot* shots, bool need_sct) {
                             }
                         }
                     }
+                    spread |= hsmp.ntaps() > t0 + 1;
                 }
                 hsmp.close_item();
             }
@@ -467,6 +481,13 @@ void SsgBase::build_tables(int S, const owl_shot* shots, bool need_sct) {
         return b > POINT_CLUSTER ? b : b > 4 ? POINT_CLUSTER : b > 2 ? 4 : b;
     };
     max_traces = mr;
+    if (spread && horg.size() == (size_t)rtot) {
+        std::vector<float> f((size_t)FW * rtot);
+        for (int r = 0; r < rtot; ++r)
+            for (int k = 0; k < FW; ++k) f[(size_t)k * rtot + r] = hfac[(size_t)r * FW + k];
+        rec_fac.upload(f.data(), f.size(), stream);
+        rec_org.upload(horg.data(), horg.size(), stream);
+    }
     nb_rec = ctas(mr);
     nb_sct = ctas(ms);
     inj.upload(hinj, stream);

@@ -112,6 +112,10 @@ struct SsgBase : Engine {
     bool taps_inside = false;  // every source tap of the batch lies on a node its kernel updates
     int max_traces = 0;        // most traces of a shot of the batch
     DevBuf<int> inj_last;      // per shot: last step (1-based) whose source amplitudes are not all zero
+    // per trace, where the medium has them (rec_window): storage coordinates (x, z) of its window's first tap, and
+    // its weight's factors, [k][trace]: BOX_W along x, BOX_W along z, the trace's weight
+    DevBuf<int2> rec_org;
+    DevBuf<float> rec_fac;
     DevBuf<unsigned char> live;
     DevBuf<long long> segbuf;  // st_segments offsets then lengths, on the device
     GraphCache g_fwd, g_rec, g_adj, g_fst;
@@ -150,6 +154,12 @@ struct SsgBase : Engine {
     virtual void src_taps(const owl_source& q, int comp, std::vector<TapPt>& taps, long long& rho_cell,
                           float& rho_val) const = 0;
     virtual void rec_taps(const owl_receiver& q, int comp, std::vector<TapPt>& taps) const = 0;
+    // the window of a trace whose taps are all BOX_W x BOX_W nodes of field 0 with weights (fx[i] fz[k]) w, rounded
+    // in this order (those of weight 0 are no taps): reference indices of its first tap, and the factors
+    virtual bool rec_window(const owl_receiver& q, int& i, int& k, float* fx, float* fz, float& w) const {
+        (void)q; (void)i; (void)k; (void)fx; (void)fz; (void)w;
+        return false;
+    }
     // adjoint of one sampling tap (free-surface images route through the mirrored node)
     virtual void scatter_map(const TapPt& t, std::vector<TapPt>& out) const { out.push_back(t); }
     virtual void launch_kernel(int id, int S, bool store) = 0;

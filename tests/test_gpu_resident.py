@@ -105,3 +105,40 @@ def test_what_stays_step_by_step():
         b = s.forward(ps, o)
         assert s.last_info.gpu_launches > 2 * nt
         np.testing.assert_array_equal(a, b)
+
+
+def spread(nx, nz, half, pml, fs, pattern):
+    """Receivers off the nodes: on every row, above a free surface, beside the sources, out to the edges of the
+    absorbing layer; `pattern` picks nodes along x, along z, both or none."""
+    ox, oz = {"x": (0.0, 3.7), "z": (4.1, 0.0), "both": (0.0, 0.0), "none": (4.1, 3.7)}[pattern]
+    lo, hi = -10.0 * min(pml - 1, 3), 10.0 * min(pml - 1, 3)
+    recs = [Receiver(x=10.0 * (nx // 3) + ox, z=10.0 * k + oz, weight=1.0 - 0.01 * (k % 5)) for k in range(nz - 1)]
+    recs += [Receiver(x=lo + ox + (10.0 * nx + hi - lo) * i / 40.0, z=30.0 + oz) for i in range(40)]
+    recs += [Receiver(x=10.0 * (nx // 2) + 13.0 * i + ox, z=(-7.0 if fs else 2.0) + oz) for i in range(-4, 5)]
+    recs += [Receiver(x=10.0 * (nx // 2) + ox, z=10.0 * nz + hi - 20.0 + oz)]
+    return recs
+
+
+@pytest.mark.parametrize("pattern", ["x", "z", "both", "none"])
+@pytest.mark.parametrize("nx,nz,pml,half,fs,nsrc", [(61, 47, 6, 4, True, 3), (64, 48, 10, 8, False, 1),
+                                                    (77, 53, 11, 8, True, 2), (131, 203, 20, 4, False, 4)])
+def test_traces_of_several_taps(nx, nz, pml, half, fs, nsrc, pattern):
+    """Windows on one CTA's rows, across two, above the surface and on the sources' taps, against the step launches."""
+    vp, rho = model(nz, nx)
+    nt = 160
+    s = SSGSolver(L.OWL_ACOUSTIC_ISO_2D, nx, nz, 10.0, 10.0, 1e-3, nt, pml=pml, fdhalf=half, free_surface=fs,
+                  f0_max=12.0, max_shots=2)
+    s.set_model(vp, rho)
+    shots = [Shot(k + 1, [Source(x=10.0 * (nx // 2) + 7.3 * j, z=52.0 + 41.0 * j, f0=14.0 + j, t0=0.03 * j)
+                          for j in range(nsrc)], spread(nx, nz, half, pml, fs, pattern)[k:]) for k in range(2)]
+    ps = s.prepare(shots)
+    a = s.forward(ps, RunOpts())
+    assert s.last_info.gpu_launches < nt
+    b = s.forward(ps, STEPWISE)
+    assert s.last_info.gpu_launches > 2 * nt
+    assert np.all(np.isfinite(b)) and np.abs(b).max() > 0
+    np.testing.assert_array_equal(a, b)
+    # the same with the traces recorded segment by segment, at the data sampling of a gradient's forward
+    syn = np.zeros_like(b)
+    s.gradient(ps, (0.5 * b).astype(np.float32), opts=RunOpts(checkpoint_interval=33), seis_out=syn)
+    np.testing.assert_array_equal(syn, b)
