@@ -611,13 +611,14 @@ def headline_roofline(s, d, k, peak, peak_kind):
     # the other segments storing; adjoint every step
     counts = {L.OWL_K_FWD_P: nt - n_last, L.OWL_K_FWD_V: nt - n_last, L.OWL_K_FWD_P_STORE: nt,
               L.OWL_K_FWD_V_STORE: nt, L.OWL_K_ADJ_P: nt, L.OWL_K_ADJ_V: nt}
-    # the forward and recomputed segments run as one launch each with the state in
-    # shared memory (no step kernels) where a gradient has about two launches per
-    # step: the adjoint's
-    resident = s.last_info.gpu_launches < 3 * nt
+    # resident segments (one launch each, the state in shared memory) run no step
+    # kernels: the run info gives the forward's CTAs per shot as a negative
+    # shots_per_cta_forward, and no forward tile where the recomputed ones run so too
+    resident = s.last_info.shots_per_cta_forward < 0
     if resident:
-        for kid in (L.OWL_K_FWD_P, L.OWL_K_FWD_V, L.OWL_K_FWD_P_STORE, L.OWL_K_FWD_V_STORE):
-            counts[kid] = 0
+        counts[L.OWL_K_FWD_P] = counts[L.OWL_K_FWD_V] = 0
+        again = nt - n_last if s.last_info.tile_z_forward != 0 else 0
+        counts[L.OWL_K_FWD_P_STORE] = counts[L.OWL_K_FWD_V_STORE] = again
     # the autotuner's variants: tile codes 100 + h are the four-cell kernels,
     # 200 + h the same with the pipelined adjoint p kernel, 300 + h the
     # one-cell kernels with it (pipelined only when a CTA takes several shots)

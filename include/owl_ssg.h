@@ -243,8 +243,10 @@ typedef struct {
     int batches;
     int checkpoint_interval;  /* gradients: the interval used (opts, or chosen from free device memory) */
     int shots_per_launch;     /* shots per batched launch used (opts, or the most that fit the device) */
-    int tile_z_forward;       /* the forward kernels' tile code (tile_z is the adjoint kernels' in a gradient) */
-    int shots_per_cta_forward; /* the forward kernels' shots per CTA (shots_per_cta is the adjoint kernels' in a gradient) */
+    int tile_z_forward;       /* the forward kernels' tile code (tile_z is the adjoint kernels' in a gradient); 0: no
+                                 step kernel ran in the forward and recomputed segments */
+    int shots_per_cta_forward; /* the forward kernels' shots per CTA (shots_per_cta is the adjoint kernels' in a gradient);
+                                  -C: the forward ran resident segments, C CTAs per shot (2D acoustic) */
 } owl_run_info;
 
 /* ---- lifecycle ---------------------------------------------------------- */

@@ -901,7 +901,7 @@ struct Ac2dEngine : SsgBase {
     DevBuf<unsigned> pbar;  // the grid barrier's arrival count and generation
     int num_sms = 0;
     bool run_steps_persistent(int kind, int n, int S) override {
-        if (kind != 2 && resident(0, S)) {
+        if (resident(kind, S)) {
             if (R == 4) launch_res<4>(kind, n, S);
             else launch_res<8>(kind, n, S);
             return true;
@@ -962,7 +962,8 @@ struct Ac2dEngine : SsgBase {
         size_t smem = 0;
         int threads = 0, H = 4;
         bool one = true;
-        double us = 0.0;  // modelled time of a step of the whole batch
+        int waves = 1;     // launches of as many clusters as fit the device at once
+        double us = 0.0;   // modelled time of a step of one wave, traces on nodes, one injection item
     };
     std::map<int, ResPlan> res_plans;  // by shots per launch
     // rows of each CTA. The slowest CTA sets the pace, and a z-PML row costs about
@@ -1018,14 +1019,31 @@ struct Ac2dEngine : SsgBase {
         return false;
     }
 
-    // cluster size: the least modelled time of a step of the batch. One CTA per SM
-    // (two on one SM took twice as long as two SMs, and clusters are packed that
-    // way unless the shared memory forbids it), about 2.1 us of barriers and phase
-    // starts per step and 0.41 ns per cell of the largest CTA (measured: 181 x 131
-    // cells on 4 / 8 / 16 CTAs 4.7 / 3.7 / 2.7 us, 441 x 241 on 16 CTAs 5.0 us),
-    // the shots in waves of as many clusters as fit the device. Every fitting size
-    // beats the step launches (8.2 and 8.8 us per step for one shot of these
-    // grids, 35.7 against 25.7 us for 32 shots of the larger).
+    // Cluster size: 1, 2, 4, 8 or 16 CTAs, the least modelled time of a step of the
+    // batch, one CTA per SM (two on one SM took twice as long as two SMs, and
+    // clusters are packed that way unless the shared memory forbids it), the shots in
+    // waves of as many clusters as fit the device. The model, us per step: 1.9 for
+    // barriers and phase starts, and for each pass of the CTA's threads over its items
+    // a part that grows with the threads (issue, shared memory). Measured against it,
+    // one shot, half-width 4: 100 x 80 on 2 / 4 / 8 / 16 CTAs 4.8 / 3.5 / 2.7 / 2.5
+    // (5.3 / 3.6 / 3.0 / 2.7), 250 x 150 and 401 x 201 on 16 4.6 / 5.5 (4.8 / 5.4), two
+    // passes: 250 x 150 on 8 8.5, 440 x 215 on 16 7.2 (8.2); half-width 8: 100 x 80 on
+    // 4 / 8 4.4 / 3.3 (5.4 / 4.3), two passes: 287 x 173 and 380 x 180 on 16 7.5 / 9.1
+    // (7.4 / 9.0). Segments that store the stencil terms take about 1.4 times that.
+    double res_model(int H, int threads, int passes) const {
+        const double per = R == 8 ? 1.3 + 0.005 * threads : H == 2 ? 0.45 + 0.0028 * threads : 1.5 + 0.0045 * threads;
+        return 1.9 + passes * (per + (passes > 1 && R == 4 ? 0.5 : 0.0));
+    }
+    // Step kernels, the same: about 9 us of three launches and, per million cells of
+    // the batch, 8.6 (half-width 4) or 9 us up to 4 million (resident in L2), 14 / 16
+    // beyond. Measured (model): 401 x 201, 8 / 16 / 32 / 64 shots 15.7 / 22.1 / 34.5 /
+    // 77 (16 / 23 / 38 / 82); half-width 8, 380 x 180, 8 / 16 / 64 15.0 / 22.7 / 89
+    // (16 / 23 / 76). Storing segments up to 1.3 times that.
+    double step_model(int S, bool store) const {
+        const double mc = 1e-6 * NXp * NZp * S, slope = R == 8 ? 9.0 : 8.6, far = R == 8 ? 16.0 : 14.0;
+        const double t = (R == 8 ? 9.5 : 8.8) + slope * std::min(mc, 4.0) + far * std::max(mc - 4.0, 0.0);
+        return store ? t * std::min(1.3, 1.0 + 0.05 * mc) : t;
+    }
     using ResKernel = void (*)(Ac2dDev, Ac2dRes);
     template <int RR>
     static ResKernel res_kernel(int H, bool store, bool one) {
@@ -1079,21 +1097,42 @@ struct Ac2dEngine : SsgBase {
                 (void)cudaGetLastError();
                 continue;
             }
-            const int waves = (S + slots - 1) / slots;
-            p.us = waves * (4.1e-4 * rows * NXp + 2.1);
+            p.waves = (S + slots - 1) / slots;
+            p.us = res_model(p.H, p.threads, passes);
             p.ok = true;
-            if (!best.ok || p.us < best.us) best = p;
+            if (!best.ok || p.waves * p.us < best.waves * best.us) best = p;
         }
         return res_plans[S] = best;
     }
-    // forward steps of the batch run resident: the automatic mode, explosion
-    // sources only (force taps enter between the velocity update and the halo
-    // exchange) whose taps lie inside the updated nodes (the arrays end there),
-    // traces that the threads of one CTA can hold
-    bool resident(int pass, int S) override {
-        if (pass != 0 || !res_allowed || fuse_fwd || !taps_inside || (inj_fmask & 6)) return false;
+    // The batch runs resident: the automatic mode, explosion sources only (force taps
+    // enter between the velocity update and the halo exchange) whose taps lie inside
+    // the updated nodes (the arrays end there), traces that the threads of one CTA can
+    // hold, and the modelled step shorter than the step kernels'. Forward segments and
+    // recomputed ones (which store) are decided apart: all forwards of a batch run
+    // alike. Many shots of a grid that takes two passes, half-width 8 above all, and
+    // storing segments of it are faster step by step (380 x 180, 16 shots, half-width
+    // 8: 22.7 against 27.0 us, storing 24.0 against 36.4; 250 x 150, 16 shots, storing
+    // 18.0 against 19.2). Windows (traces of several taps) cost a wave 0.4 us and, while
+    // the sources are active, 1.2 and 0.0025 per trace, the step kernels 5 us and 0.012
+    // per trace; injection items past the first, while active, 1.7 us a wave and 0.33
+    // each, against 0.6 each. Near a tie the resident kernel is taken (8 %, the models'
+    // error; it needs no tuning). Over 139 grids, shot counts, trace and source
+    // layouts the chosen path took 0.5 % longer than the better one, 13 % at the worst.
+    bool resident(int kind, int S) override {
+        if (kind == 2 || !res_allowed || fuse_fwd || !taps_inside || (inj_fmask & 6)) return false;
         const ResPlan& p = R == 4 ? res_plan<4>(S) : res_plan<8>(S);
-        return p.ok && max_traces <= 2 * p.threads;
+        if (!p.ok || max_traces > 2 * p.threads) return false;
+        const bool store = kind == 1, sample = kind != 1;
+        double res = p.us * (store ? 1.4 : 1.0), step = step_model(S, store);
+        if (sample && windows) {
+            res += 0.4 + inj_active * (1.2 + 0.0025 * max_traces);
+            step += 5.0 + 0.012 * max_traces;
+        }
+        if (max_items > 1) {
+            res += inj_active * (1.7 + 0.33 * (max_items - 1));
+            step += inj_active * 0.6 * (max_items - 1);
+        }
+        return 0.92 * p.waves * res < step;
     }
     template <int RR>
     void launch_res(int kind, int n, int S) {
@@ -1118,6 +1157,7 @@ struct Ac2dEngine : SsgBase {
         cfg.stream = stream;
         OWL_CUDA(cudaLaunchKernelEx(&cfg, k, a, q));
         launches++;
+        if (kind != 1) res_ctas = q.C;
     }
 
     // compulsory bytes of one launch (each state field read / written once per

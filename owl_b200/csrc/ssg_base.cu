@@ -371,7 +371,7 @@ void SsgBase::build_tables(int S, const owl_shot* shots, bool need_sct) {
     std::vector<int2> horg;       // windows of the traces and their factors, FW floats a trace
     std::vector<float> hfac;
     constexpr int FW = 2 * BOX_W + 1;
-    bool spread = false;          // some trace has more than one tap
+    windows = false;
     rtot = 0;
     for (int s = 0; s < S; ++s) {
         const owl_shot& sh = shots[s];
@@ -451,7 +451,7 @@ void SsgBase::build_tables(int S, const owl_shot* shots, bool need_sct) {
                             }
                         }
                     }
-                    spread |= hsmp.ntaps() > t0 + 1;
+                    windows |= hsmp.ntaps() > t0 + 1;
                 }
                 hsmp.close_item();
             }
@@ -472,6 +472,9 @@ void SsgBase::build_tables(int S, const owl_shot* shots, bool need_sct) {
             for (int t = nt; t > hlast[s]; --t)
                 if (hamp[(size_t)it * nt + t - 1] != 0.f) hlast[s] = t;
     inj_last.upload(hlast.data(), hlast.size(), stream);
+    inj_active = (double)*std::max_element(hlast.begin(), hlast.end()) / nt;
+    max_items = 0;
+    for (int s = 0; s < S; ++s) max_items = std::max(max_items, hinj_ptr[s + 1] - hinj_ptr[s]);
     int mr = 0, ms = 0;
     for (size_t i = 0; i + 1 < hrec_ptr.size(); ++i) mr = std::max(mr, hrec_ptr[i + 1] - hrec_ptr[i]);
     for (size_t i = 0; i + 1 < hsct_ptr.size(); ++i) ms = std::max(ms, hsct_ptr[i + 1] - hsct_ptr[i]);
@@ -481,7 +484,7 @@ void SsgBase::build_tables(int S, const owl_shot* shots, bool need_sct) {
         return b > POINT_CLUSTER ? b : b > 4 ? POINT_CLUSTER : b > 2 ? 4 : b;
     };
     max_traces = mr;
-    if (spread && horg.size() == (size_t)rtot) {
+    if (windows && horg.size() == (size_t)rtot) {
         std::vector<float> f((size_t)FW * rtot);
         for (int r = 0; r < rtot; ++r)
             for (int k = 0; k < FW; ++k) f[(size_t)k * rtot + r] = hfac[(size_t)r * FW + k];
@@ -617,6 +620,7 @@ void SsgBase::launch_step(int kind, int S, const PointDev& q) {
 void SsgBase::run_steps(int kind, int n, int S, const PointDev& q, bool graph) {
     if (n <= 0) return;
     if (run_steps_persistent(kind, n, S)) return;
+    res_steps |= kind != 2;
     if (!graph) {
         for (int i = 0; i < n; ++i) launch_step(kind, S, q);
         OWL_LAUNCH_CHECK();
@@ -732,6 +736,8 @@ void SsgBase::resolve_opts(const owl_run_opts& o, int nshots, const owl_shot* sh
     spt_f = spt_a = std::min(o.shots_per_cta > 0 ? o.shots_per_cta : 1, B);
     graph = o.use_graph >= 0;
     res_allowed = tune && graph;
+    res_ctas = 0;
+    res_steps = false;
     launch_params(o);
 }
 
@@ -770,7 +776,7 @@ void SsgBase::autotune(int S, int k, bool grad, bool all) {
             tz_x = it->second[1];
             continue;
         }
-        if (!all && resident(pass, S)) continue;
+        if (!all && (pass == 0 ? resident(0, S) && (!grad || resident(1, S)) : resident(2, S))) continue;
         set_step(k);
         const std::vector<int> tzs = tune_tz(pass);
         float best = 1e30f;
@@ -904,6 +910,14 @@ void SsgBase::fill_info(owl_run_info& info, int nshots, int batches, bool grad) 
     info.shots_per_launch = plan_B;
     info.tile_z_forward = tz_f;
     info.shots_per_cta_forward = spt_f;
+    if (res_ctas > 0) {
+        info.shots_per_cta_forward = -res_ctas;
+        info.tile_z_forward = res_steps ? tz_f : 0;
+        if (!grad) {
+            info.shots_per_cta = info.shots_per_cta_forward;
+            info.tile_z = info.tile_z_forward;
+        }
+    }
 }
 
 void SsgBase::forward(int nshots, const owl_shot* shots, const owl_run_opts& o, float* seis, int mem,

@@ -111,6 +111,11 @@ struct SsgBase : Engine {
     bool res_allowed = false;  // this call may run whole segments as one launch (automatic tiles, graphs on)
     bool taps_inside = false;  // every source tap of the batch lies on a node its kernel updates
     int max_traces = 0;        // most traces of a shot of the batch
+    int max_items = 0;         // most injection items of a shot of the batch
+    bool windows = false;      // some trace of the batch has several taps (rec_org, rec_fac are its windows)
+    double inj_active = 0.0;   // share of the steps with a nonzero source amplitude
+    int res_ctas = 0;          // CTAs per shot of the call's resident forward segments (0: step by step)
+    bool res_steps = false;    // the call ran forward or recomputed segments step by step
     DevBuf<int> inj_last;      // per shot: last step (1-based) whose source amplitudes are not all zero
     // per trace, where the medium has them (rec_window): storage coordinates (x, z) of its window's first tap, and
     // its weight's factors, [k][trace]: BOX_W along x, BOX_W along z, the trace's weight
@@ -224,10 +229,10 @@ struct SsgBase : Engine {
         (void)kind; (void)n; (void)S;
         return false;
     }
-    // whether the medium runs the forward (pass 0) / adjoint (pass 1) steps of a
-    // batch of S shots as one launch per segment (automatic mode)
-    virtual bool resident(int pass, int S) {
-        (void)pass; (void)S;
+    // whether the medium runs the steps of `kind` (launch_step) of a batch of S
+    // shots as one launch per segment (automatic mode)
+    virtual bool resident(int kind, int S) {
+        (void)kind; (void)S;
         return false;
     }
     void run_steps(int kind, int n, int S, const PointDev& q, bool graph);

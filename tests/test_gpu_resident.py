@@ -142,3 +142,38 @@ def test_traces_of_several_taps(nx, nz, pml, half, fs, nsrc, pattern):
     syn = np.zeros_like(b)
     s.gradient(ps, (0.5 * b).astype(np.float32), opts=RunOpts(checkpoint_interval=33), seis_out=syn)
     np.testing.assert_array_equal(syn, b)
+
+
+@pytest.mark.parametrize("nx,nz,pml,half,nshots,forward,again", [
+    (100, 80, 10, 4, 3, True, True),      # one wave
+    (250, 150, 20, 4, 16, True, False),   # three waves: the storing segments are faster step by step
+    (380, 180, 20, 8, 16, False, False),  # two passes a thread, three waves
+])
+def test_which_segments_run_resident(nx, nz, pml, half, nshots, forward, again):
+    """Forward and recomputed segments are chosen apart; the run info tells which ran, and the results agree."""
+    vp, rho = model(nz, nx)
+    nt = 60
+    s = SSGSolver(L.OWL_ACOUSTIC_ISO_2D, nx, nz, 10.0, 10.0, 1e-3, nt, pml=pml, fdhalf=half, f0_max=12.0,
+                  max_shots=nshots)
+    s.set_model(vp, rho)
+    ps = s.prepare([Shot(k + 1, [Source(x=10.0 * nx * (k + 1) / (nshots + 1) + 3.3, z=61.7, f0=12.0)],
+                         [Receiver(x=20.0 * i + 20.0, z=20.0) for i in range(20)]) for k in range(nshots)])
+    b = s.forward(ps, STEPWISE)
+    assert s.last_info.shots_per_cta_forward == 1 and s.last_info.tile_z_forward == 8
+    a = s.forward(ps, RunOpts())
+    info = s.last_info
+    assert (info.shots_per_cta_forward < 0, info.gpu_launches < nt) == (forward, forward)
+    if forward:
+        np.testing.assert_array_equal(a, b)
+        assert info.tile_z_forward == 0 and (info.tile_z, info.shots_per_cta) == (0, info.shots_per_cta_forward)
+    else:
+        close(a, b)
+    obs = (0.5 * b).astype(np.float32)
+    syn = np.zeros_like(b)
+    _, g0 = s.gradient(ps, obs, opts=RunOpts(checkpoint_interval=20), seis_out=syn)
+    assert (s.last_info.shots_per_cta_forward < 0) == forward
+    assert (s.last_info.tile_z_forward == 0) == again
+    np.testing.assert_array_equal(syn, a)  # the forward of a gradient runs as a forward alone
+    _, g1 = s.gradient(ps, obs, opts=RunOpts(checkpoint_interval=20, use_graph=-1, tile_z=8, shots_per_cta=1))
+    for p in range(2):
+        close(np.split(g0, 2)[p], np.split(g1, 2)[p])
