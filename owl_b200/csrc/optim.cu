@@ -38,6 +38,11 @@ constexpr int RED_BLOCKS = 148 * 8;
 // and an update per pair were 6 np + 4 launches and 2 np + 1 host waits. A field
 // of 80 k cells is latency bound: 401 x 201, six models, smoothing and taper
 // included, takes 0.15 ms a pass against 2.1 ms (with the workspaces of workspace.cuh).
+// A large field is bound by HBM, which needs some 40 KB of reads in flight per SM:
+// a thread takes LB_CELLS cells at once, on up to four blocks of an SM. Six models of
+// 12 / 40 / 85 million cells take 0.61 / 1.83 / 3.80 ms (6.1 TB/s), with one cell at a
+// time on two blocks 1.65 / 5.2 / 11.0, with the launches that waited for the host
+// 2.4 / 4.5 / 7.6; eight blocks gain 2 % there and lose 27 % on 361 k cells.
 struct LbStep {
     long long n;
     int nparts;               // blocks of the launch before (its partials), 0: none
@@ -50,6 +55,7 @@ struct LbStep {
     const float *u1, *u0;     // update vector u1 - u0 of pair prev
     const float *x1, *x0, *g1, *g0;  // next pair: s = x1 - x0, y = g1 - g0
 };
+constexpr int LB_CELLS = 4;
 enum { LB_FIRST = 0, LB_DOWN, LB_TURN, LB_UP, LB_LAST };
 
 // sums of three values over the block (256 threads, fixed order), in every thread
@@ -111,23 +117,48 @@ __global__ void __launch_bounds__(256) k_lbfgs(const __grid_constant__ LbStep a)
         }
     }
     double p0 = 0.0, p1 = 0.0, p2 = 0.0;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += (long long)gridDim.x * blockDim.x) {
-        float q = a.src[i];
-        if (MODE != LB_FIRST) {
-            q = (float)((double)q + coef * ((double)a.u1[i] - (double)a.u0[i]));
-            if (MODE == LB_TURN) q = (float)(gamma * (double)q);
-            if (MODE == LB_LAST) q = -q;
+    // LB_CELLS cells a thread at once, their reads ahead of their writes (r may be src)
+    const long long step = (long long)gridDim.x * blockDim.x;
+    for (long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x; i0 < a.n; i0 += LB_CELLS * step) {
+        float q[LB_CELLS], u1[LB_CELLS], u0[LB_CELLS], x1[LB_CELLS], x0[LB_CELLS], g1[LB_CELLS], g0[LB_CELLS];
+#pragma unroll
+        for (int e = 0; e < LB_CELLS; ++e) {
+            const long long i = i0 + e * step;
+            if (i >= a.n) continue;
+            q[e] = a.src[i];
+            if (MODE != LB_FIRST) {
+                u1[e] = a.u1[i];
+                u0[e] = a.u0[i];
+            }
+            if (MODE == LB_FIRST || MODE == LB_DOWN) {
+                x1[e] = a.x1[i];
+                x0[e] = a.x0[i];
+            }
+            if (MODE != LB_LAST) {
+                g1[e] = a.g1[i];
+                g0[e] = a.g0[i];
+            }
         }
-        if (MODE != LB_FIRST) a.r[i] = q;
-        if (MODE == LB_LAST) continue;
-        const double y = (double)a.g1[i] - (double)a.g0[i];
-        if (MODE == LB_FIRST || MODE == LB_DOWN) {
-            const double s = (double)a.x1[i] - (double)a.x0[i];
-            p0 += s * (double)q;
-            p1 += y * s;
-            if (MODE == LB_FIRST) p2 += y * y;
-        } else {
-            p2 += y * (double)q;
+#pragma unroll
+        for (int e = 0; e < LB_CELLS; ++e) {
+            const long long i = i0 + e * step;
+            if (i >= a.n) continue;
+            if (MODE != LB_FIRST) {
+                q[e] = (float)((double)q[e] + coef * ((double)u1[e] - (double)u0[e]));
+                if (MODE == LB_TURN) q[e] = (float)(gamma * (double)q[e]);
+                if (MODE == LB_LAST) q[e] = -q[e];
+                a.r[i] = q[e];
+            }
+            if (MODE == LB_LAST) continue;
+            const double y = (double)g1[e] - (double)g0[e];
+            if (MODE == LB_FIRST || MODE == LB_DOWN) {
+                const double s = (double)x1[e] - (double)x0[e];
+                p0 += s * (double)q[e];
+                p1 += y * s;
+                if (MODE == LB_FIRST) p2 += y * y;
+            } else {
+                p2 += y * (double)q[e];
+            }
         }
     }
     if (MODE == LB_LAST) return;
@@ -328,8 +359,8 @@ void search_direction(int method, long long n, int nm, const float* const* x, co
                       const float* prev_srch, float* srch, Workspace& ws) {
     cudaStream_t s = ws.s;
     const float* gk = g[nm - 1];
-    // two blocks per SM at most: every launch sums the partials of the one before
-    const int nb = (int)std::max<long long>(1, std::min<long long>((n + 255) / 256, 2 * 148));
+    // four blocks per SM at most: every launch sums the partials of the one before
+    const int nb = (int)std::max<long long>(1, std::min<long long>((n + 255) / 256, 4 * 148));
     if (method == OWL_SEARCH_SD || nm < 2) {
         k_negate<<<nb, 256, 0, s>>>(n, gk, srch);
         OWL_LAUNCH_CHECK();

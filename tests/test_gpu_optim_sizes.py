@@ -50,3 +50,12 @@ def test_smoothing_forms(shape, sigma):
         ref = sum(w[k] * np.take(p, range(k, k + shape[ax]), axis=ax) for k in range(2 * rad + 1))
     got = process(f, L.OWL_GRAD_SMOOTH, list(sigma))
     assert rel(got, ref) < 2e-6, rel(got, ref)
+
+
+@pytest.mark.parametrize("n", [4 * 148 * 256 - 1, 4 * 148 * 256 + 1, 4 * 4 * 148 * 256 + 300])
+@pytest.mark.parametrize("nm", [2, 4])
+def test_several_cells_per_thread(n, nm):
+    """one cell less and more than the grid's threads, and more than they take in one round"""
+    x, g = _history(n, nm, seed=n + nm)
+    ref = O.search_direction(L.OWL_SEARCH_LBFGS, x, g, None)
+    assert rel(search_direction(L.OWL_SEARCH_LBFGS, x, g), ref) < 1e-5
