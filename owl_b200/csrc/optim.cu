@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(256) k_cg_dots(long long n, const float* __res
     }
 }
 __global__ void __launch_bounds__(256) k_cg_apply(long long n, const double* __restrict__ part, int nparts,
-                                                  const float* __restrict__ g, const float* prev, float* srch) {
+                                                  const float* g, const float* prev, float* srch) {
     pdl_prologue();
     double s1, s2, z;
     sum_parts(part, nparts, s1, s2, z);
@@ -196,7 +196,8 @@ __global__ void __launch_bounds__(256) k_cg_apply(long long n, const double* __r
         srch[i] = (float)(-(double)g[i] + beta * (double)prev[i]);
 }
 
-__global__ void k_negate(long long n, const float* __restrict__ g, float* __restrict__ r) {
+// (r may be g)
+__global__ void k_negate(long long n, const float* g, float* r) {
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         r[i] = -g[i];
 }
