@@ -97,8 +97,9 @@ void launch_pdl(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStr
     launch_pdl_cluster(k, grid, block, dim3(1, 1, 1), smem, s, args...);
 }
 
-// frees the idle workspaces of the current device (workspace.cu)
+// frees the idle workspaces of the current device (workspace.cu); the bytes they hold
 void workspace_trim();
+size_t workspace_idle_bytes();
 
 // ----------------------------------------------------------------------------
 // grow-only device buffer. Keeping the pointer stable across calls lets the

@@ -687,7 +687,8 @@ double SsgBase::held_bytes() const {
 // longest interval that fits. "Fit" counts every buffer of the batch (state,
 // adjoint state, Kahan sums, the segment's stencil terms, checkpoints, traces)
 // against 92 % of the free device memory plus what the handle already holds
-// (OWL_MEM_BUDGET_MB in the environment caps that figure).
+// (OWL_MEM_BUDGET_MB in the environment caps that figure); the idle workspaces
+// count as free, since an allocation that runs out of memory releases them.
 void SsgBase::resolve_opts(const owl_run_opts& o, int nshots, const owl_shot* shots, bool grad, int& B, int& k,
                            bool& graph) {
     // tile_z: 0 = autotuned; > 0 explicit tile height (3D forward: rows per
@@ -702,7 +703,7 @@ void SsgBase::resolve_opts(const owl_run_opts& o, int nshots, const owl_shot* sh
     for (int i = 0; i < nshots && shots; ++i) recs = std::max(recs, shots[i].nrec);
     size_t fr = 0, tot = 0;
     OWL_CUDA(cudaMemGetInfo(&fr, &tot));
-    double budget = 0.92 * (double)fr + held_bytes();
+    double budget = 0.92 * ((double)fr + (double)workspace_idle_bytes()) + held_bytes();
     if (const char* e = std::getenv("OWL_MEM_BUDGET_MB")) budget = std::min(budget, std::atof(e) * 1048576.0);
     const bool auto_k = o.checkpoint_interval < 0;
     const int k_fixed = std::min(o.checkpoint_interval > 0 ? o.checkpoint_interval : 50, desc.nt);

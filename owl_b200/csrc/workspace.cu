@@ -83,6 +83,17 @@ WorkspaceLease::~WorkspaceLease() {
     delete w;
 }
 
+size_t workspace_idle_bytes() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    const unsigned long long ctx = context_id();
+    std::lock_guard<std::mutex> g(ws_lock());
+    size_t n = 0;
+    for (const Workspace* p : ws_idle())
+        if (p->dev == dev && p->ctx == ctx) n += p->held();
+    return n;
+}
+
 void workspace_trim() {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return;
