@@ -20,19 +20,22 @@ void set_last_error(const std::string& msg) { g_last_error = msg; }
 
 template <typename F>
 static int guarded(F&& f) {
+    int code = OWL_OK;
     try {
         f();
-        return OWL_OK;
     } catch (const OwlError& e) {
         set_last_error(e.what());
-        return e.code;
+        code = e.code;
     } catch (const std::bad_alloc&) {
         set_last_error("host allocation failed");
-        return OWL_ERR_OOM;
+        code = OWL_ERR_OOM;
     } catch (const std::exception& e) {
         set_last_error(e.what());
-        return OWL_ERR_INVALID;
+        code = OWL_ERR_INVALID;
     }
+    // what failed on the way (buffers given back included) is this call's error, not the next one's
+    if (code != OWL_OK) (void)cudaGetLastError();
+    return code;
 }
 
 static void check_device() {
