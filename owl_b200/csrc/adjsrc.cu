@@ -44,6 +44,8 @@ int next_power_235(int n) {
 namespace {
 
 constexpr int MAX_DFT_M = 16384;  // 128 KB of float2 work in shared memory
+// the kernels' limit, the same in every call: calls of several threads may run side by side
+constexpr int DFT_SMEM = MAX_DFT_M * (int)sizeof(float2);
 
 void host_fft(std::vector<std::complex<double>>& a) {
     const size_t M = a.size();
@@ -788,7 +790,7 @@ void AdjointSource::run(const owl_misfit_opts& o, int ngather, const int* h_gath
         la.sigma = (o.lawi_sigma > 0.f ? o.lawi_sigma : 0.25f) / o.dt;
         const size_t smem = (size_t)awl.M * sizeof(float2);
         auto k = loc ? k_adjsrc_local : k_adjsrc_spacetime;
-        OWL_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        OWL_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, DFT_SMEM));
         int per_sm = 0, nsm = 0, dev_id = 0;
         OWL_CUDA(cudaGetDevice(&dev_id));
         OWL_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev_id));
@@ -849,7 +851,7 @@ void AdjointSource::run(const owl_misfit_opts& o, int ngather, const int* h_gath
         a.deconv_eps = o.deconv_eps > 0.f ? o.deconv_eps : 0.1f;
     }
     const size_t smem = (size_t)M * sizeof(float2);
-    OWL_CUDA(cudaFuncSetAttribute(k_adjsrc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(smem, 1)));
+    OWL_CUDA(cudaFuncSetAttribute(k_adjsrc, cudaFuncAttributeMaxDynamicSharedMemorySize, DFT_SMEM));
     int per_sm = 0, nsm = 0, dev_id = 0;
     OWL_CUDA(cudaGetDevice(&dev_id));
     OWL_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev_id));
