@@ -57,10 +57,11 @@ __device__ __forceinline__ void pdl_prologue() {
 }
 
 // barrier over the CTAs of a thread-block cluster: what every thread wrote
-// before it (global or shared memory) is visible to every thread after it
+// before it (global or shared memory) is visible to every thread after it (not the
+// .aligned form: the threads of a warp may come from loops of different lengths)
 __device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
 
 bool pdl_enabled();
