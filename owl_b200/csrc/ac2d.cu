@@ -1143,7 +1143,7 @@ struct Ac2dEngine : SsgBase {
         q.smp = kind != 1;
         q.inj_last = inj_last.p;
         q.org = rec_org.p;
-        q.fac = rec_fac.p;
+        q.fac = windows && q.smp ? rec_fac.p : nullptr;
         const bool store = kind == 1 || kind == 3;
         const ResKernel k = res_kernel<RR>(p.H, store, p.one);
         cudaLaunchConfig_t cfg = {};

@@ -47,6 +47,7 @@ struct Ac2dRes {
     const int* inj_last;   // per shot: last step (1-based) with a nonzero amplitude
     const int2* org;       // traces of several taps: storage (x, z) of the window's first tap
     const float* fac;      // and the factors of its weights, [k][trace]: BOX_W along x, BOX_W along z, the trace's weight
+                           // (null where no such trace is recorded)
 };
 
 __device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -227,7 +228,10 @@ __device__ float res_read_p(const Ac2dDev& a, const Ac2dRes& q, const ResCta<R>&
 // one trace of the shot at step index cur (0-based): p plus the pending
 // explosion taps, each trace a sequential sum over its taps
 template <int R>
-__device__ __noinline__ float res_sample(const Ac2dDev& a, const Ac2dRes& q, ResCta<R> c, int r, bool pend, int cur) {
+__device__ __noinline__ float res_sample(const Ac2dDev& a, const Ac2dRes& q, int r, bool pend, int cur) {
+    extern __shared__ __align__(16) float res_sm[];
+    ResCta<R> c;
+    res_setup<R>(a, q, res_sm, c);
     float acc = 0.f;
     for (int j = a.pt.smp.ptr[r]; j < a.pt.smp.ptr[r + 1]; ++j) {
         const long long off = a.pt.smp.off[j];
@@ -268,7 +272,10 @@ __device__ __forceinline__ ResTap res_tap(const Ac2dDev& a, const Ac2dRes& q, co
 }
 // items it0 and on of step index ti (0-based), in order
 template <int R>
-__device__ __noinline__ void res_inject_items(const Ac2dDev& a, const Ac2dRes& q, ResCta<R> c, int it0, int ti, bool halo) {
+__device__ __noinline__ void res_inject_items(const Ac2dDev& a, const Ac2dRes& q, int it0, int ti, bool halo) {
+    extern __shared__ __align__(16) float res_sm[];
+    ResCta<R> c;
+    res_setup<R>(a, q, res_sm, c);
     const int end = a.pt.item_ptr[c.s + 1], nt = a.pt.nt;
     const float* amp = a.pt.amp + ti;
     ResTap t = res_tap<R>(a, q, c, it0, halo);
@@ -304,7 +311,7 @@ __device__ __forceinline__ void res_inject(const Ac2dDev& a, const Ac2dRes& q, c
     if (ti + 1 > src.last) return;
     if (src.t.o >= 0 && src.A != 0.f) c.p[src.t.o] = c.p[src.t.o] + src.A * src.t.w;
     __syncthreads();
-    if (src.nit > 1) res_inject_items<R>(a, q, c, src.it + 1, ti, src.halo);
+    if (src.nit > 1) res_inject_items<R>(a, q, src.it + 1, ti, src.halo);
 }
 
 // Receivers of the CTA, up to two per thread, found once per launch (`list`:
@@ -312,14 +319,19 @@ __device__ __forceinline__ void res_inject(const Ac2dDev& a, const Ac2dRes& q, c
 // its row, one of several to the CTA of its window's middle row: the window then
 // lies on the CTA's rows and its halo rows, which hold p of the same step from the
 // end of the P phase on.
-enum { RES_NONE = 0, RES_TAP, RES_BOX, RES_NEAR, RES_SPAN };
-struct ResRec {
-    int kind;  // one tap / a window on the CTA's own and halo rows / one that meets the taps of the shot's sources /
-               // taps beyond the CTA's rows
-    int r;     // trace
-    int o;     // shared offset of the tap, or of the window's first one
-    float w;   // the tap's weight
+struct ResRec {  // a trace of one tap on the CTA's rows
+    int r;       // trace
+    int o;       // shared offset of the tap (-1: none)
+    float w;
 };
+enum { RES_NONE = 0, RES_BOX, RES_NEAR, RES_SPAN };
+struct ResWin {  // the others (by address: a step reads them only where there are some)
+    int kind[2];  // a window on the CTA's own and halo rows / one that meets the taps of the shot's sources / taps
+                  // beyond the CTA's rows
+    int r[2];     // trace
+    int o[2];     // shared offset of the window's first tap
+};
+enum { RES_HAS_TAPS = 1, RES_HAS_NEAR = 2 };
 // halo rows of p below the CTA's last row that hold p
 template <int R>
 constexpr int RES_BELOW = R < BOX_W / 2 + 1 ? R : R - 1;
@@ -328,13 +340,18 @@ __device__ __forceinline__ int res_local(const Ac2dDev& a, const Ac2dRes& q, con
     const int z = (int)(off / a.pitch), x = (int)(off - (long long)z * a.pitch), l = z - q.zlo - c.l0;
     return l >= 0 && l < c.nr && x >= a.x0 && x < a.x1 ? (l + R) * q.XP + (x - a.x0) + R : -1;
 }
+// (returns RES_HAS_*: some thread of the CTA has a trace of one tap / some window of
+// the shot, on whichever CTA, meets the taps of its sources)
 template <int R>
-__device__ __forceinline__ bool res_find_receivers(const Ac2dDev& a, const Ac2dRes& q, const ResCta<R>& c, int* list,
-                                                   ResRec (&rec)[2]) {
+__device__ __noinline__ int res_find_receivers(const Ac2dDev& a, const Ac2dRes& q, ResRec* rec, ResWin* win) {
+    extern __shared__ __align__(16) float res_sm[];
+    ResCta<R> c;
+    res_setup<R>(a, q, res_sm, c);
+    int* list = reinterpret_cast<int*>(res_sm);
     if (threadIdx.x == 0) list[0] = 0;
     __syncthreads();
     const Ac2dPt& t = a.pt;
-    bool near = false;  // some window of the shot, on whichever CTA, meets the taps of its sources
+    bool near = false;
     if (q.smp)
         for (int r = t.rec_ptr[c.s] + threadIdx.x; r < t.rec_ptr[c.s + 1]; r += blockDim.x) {
             const int j = t.smp.ptr[r], n = t.smp.ptr[r + 1] - j;
@@ -350,29 +367,30 @@ __device__ __forceinline__ bool res_find_receivers(const Ac2dDev& a, const Ac2dR
         }
     __syncthreads();
     const int count = list[0];
-#pragma unroll
     for (int e = 0; e < 2; ++e) {
         const int k = threadIdx.x + e * blockDim.x;
-        rec[e].kind = RES_NONE;
+        rec[e] = ResRec{0, -1, 0.f};
+        win->kind[e] = RES_NONE;
         if (k < count) {
-            const int r = list[1 + k];
-            const int j = t.smp.ptr[r];
-            rec[e].r = r;
+            const int r = list[1 + k], j = t.smp.ptr[r];
+            win->r[e] = rec[e].r = r;
             if (t.smp.ptr[r + 1] == j + 1) {
                 rec[e].w = t.smp.w[j];
                 rec[e].o = res_local<R>(a, q, c, t.smp.off[j]);
-                rec[e].kind = rec[e].o >= 0 ? RES_TAP : RES_SPAN;
+                if (rec[e].o < 0) win->kind[e] = RES_SPAN;
             } else {
                 const int2 g = q.org[r];
                 const int l = g.y - q.zlo - c.l0, x = g.x - a.x0;
-                rec[e].o = (l + R) * q.XP + x + R;
-                rec[e].kind = l < -R || l + BOX_W > c.nr + RES_BELOW<R> || x < -R || x + BOX_W > 4 * q.XG + R ? RES_SPAN
-                              : ac2d_inj_near(t, c.s, 1, g.x, g.x + BOX_W, g.y, g.y + BOX_W)                  ? RES_NEAR
-                                                                                                              : RES_BOX;
+                win->o[e] = (l + R) * q.XP + x + R;
+                win->kind[e] = l < -R || l + BOX_W > c.nr + RES_BELOW<R> || x < -R || x + BOX_W > 4 * q.XG + R ? RES_SPAN
+                               : ac2d_inj_near(t, c.s, 1, g.x, g.x + BOX_W, g.y, g.y + BOX_W)                  ? RES_NEAR
+                                                                                                               : RES_BOX;
             }
         }
     }
-    return __syncthreads_or(near);
+    const bool taps = __syncthreads_or(rec[0].o >= 0 || rec[1].o >= 0);
+    near = __syncthreads_or(near);
+    return (taps ? RES_HAS_TAPS : 0) | (near ? RES_HAS_NEAR : 0);
 }
 // a trace of several taps from the CTA's own and halo rows: the taps in order (z
 // outer), weight by weight as the tables have them. The window's values lie at
@@ -404,17 +422,27 @@ __device__ __noinline__ float res_box(const float* __restrict__ f, int n, int XP
     }
     return acc;
 }
-// record the CTA's traces of one tap, and with `near` those whose windows meet the
-// sources' taps, from p with the step's injection (halo rows included then), as
-// trace row `row`; complete (for every thread) after it
-__device__ __forceinline__ void res_record(const Ac2dDev& a, const Ac2dRes& q, const float* p, const ResRec (&rec)[2],
-                                           int row, bool near) {
-#pragma unroll
+// the thread's traces of several taps at row `row`: from the V phase's p (halo rows
+// complete), except those that meet the taps of an active source (pend), and after
+// the injection into own and halo rows (met) only those
+template <int R>
+__device__ __noinline__ void res_windows(const Ac2dDev& a, const Ac2dRes& q, const ResWin* win, int row, bool pend,
+                                         bool met) {
     for (int e = 0; e < 2; ++e) {
-        float* out = a.pt.rec + (size_t)row * a.pt.rtot + rec[e].r;
-        if (rec[e].kind == RES_TAP) *out = 0.f + p[rec[e].o] * rec[e].w;
-        if (near && rec[e].kind == RES_NEAR) *out = res_box(q.fac + rec[e].r, a.pt.rtot, q.XP, rec[e].o);
+        const int kind = win->kind[e], r = win->r[e];
+        float* out = a.pt.rec + (size_t)row * a.pt.rtot + r;
+        if (met ? kind == RES_NEAR : kind == RES_BOX || (kind == RES_NEAR && !pend))
+            *out = res_box(q.fac + r, a.pt.rtot, q.XP, win->o[e]);
+        else if (!met && kind == RES_SPAN)
+            *out = res_sample<R>(a, q, r, pend, row - 1);
     }
+}
+// record the CTA's traces of one tap, from p with the step's injection, as trace
+// row `row`; complete (for every thread) after it
+__device__ __forceinline__ void res_record(const Ac2dDev& a, const float* p, const ResRec (&rec)[2], int row) {
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+        if (rec[e].o >= 0) a.pt.rec[(size_t)row * a.pt.rtot + rec[e].r] = 0.f + p[rec[e].o] * rec[e].w;
     __syncthreads();
 }
 
@@ -547,10 +575,10 @@ __device__ __forceinline__ ResItem<R, H> res_item(const Ac2dDev& a, const Ac2dRe
         if (!(a.fsurf && c.rank == 0 && l == 0)) t.live |= 1u << h;
         if (c.pz_i(l)) t.pi |= 1u << h;
         if (c.pz_h(l)) t.ph |= 1u << h;
-        // p: my rows 0 .. R - 2 follow the CTA above (at half-width 4 row R - 1 too, for its traces' windows), my
+        // p: my rows 0 .. R - 2 follow the CTA above (where traces have windows, all rows that those may reach), my
         // last R rows precede the CTA below;
         // vz: my rows 0 .. R - 1 follow the CTA above, my last R - 1 rows precede the CTA below
-        if (c.rank > 0 && l < RES_BELOW<R>) t.up |= 1u << h;
+        if (c.rank > 0 && l < (q.fac ? RES_BELOW<R> : R - 1)) t.up |= 1u << h;
         if (c.rank > 0 && l < R) t.uv |= 1u << h;
         if (c.rank + 1 < q.C && l >= c.nr - R) t.dp |= 1u << h;
         if (c.rank + 1 < q.C && l > c.nr - R) t.dv |= 1u << h;
@@ -766,9 +794,12 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_ac2d_fwd_res(const __grid_co
     ResCta<R> c;
     res_setup<R>(a, q, res_sm, c);
     const int cur0 = *a.d_step;
-    ResRec rec[2];
-    const bool near = res_find_receivers<R>(a, q, c, reinterpret_cast<int*>(res_sm), rec);
-    const bool taps = __syncthreads_or(rec[0].kind == RES_TAP || rec[1].kind == RES_TAP);
+    ResRec found[2];
+    ResWin win;
+    const int has = res_find_receivers<R>(a, q, found, &win);
+    const ResRec rec[2] = {found[0], found[1]};
+    const bool taps = has & RES_HAS_TAPS, near = has & RES_HAS_NEAR;
+    const bool wins = win.kind[0] != RES_NONE || win.kind[1] != RES_NONE;  // the thread has traces of several taps
     ResSrc src;
     res_find_source<R>(a, q, c, near, src);
     const float* amp = a.pt.amp + (size_t)src.it * a.pt.nt;
@@ -799,8 +830,9 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_ac2d_fwd_res(const __grid_co
         if (i > 0) {
             const bool meet = near && cur <= src.last;
             res_inject<R>(a, q, c, src, cur - 1);
-            if (taps || meet) res_record(a, q, c.p, rec, cur, meet);
+            if (taps) res_record(a, c.p, rec, cur);
             if (meet) {
+                if (wins) res_windows<R>(a, q, &win, cur, true, true);
                 cluster_arrive();
                 cluster_wait();
             }
@@ -816,18 +848,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_ac2d_fwd_res(const __grid_co
         cluster_arrive();
         if (cur + 1 <= src.last && src.nit > 0) src.A = __ldg(amp + cur);
         cluster_wait();
-        // receivers of several taps or of other CTAs' nodes, from p and the pending taps of this step
-        if (cur + 2 <= a.pt.nt) {
-            const bool pend = cur + 1 <= src.last;
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                float* out = a.pt.rec + (size_t)(cur + 1) * a.pt.rtot + rec[e].r;
-                if (rec[e].kind == RES_BOX || (rec[e].kind == RES_NEAR && !pend))
-                    *out = res_box(q.fac + rec[e].r, a.pt.rtot, q.XP, rec[e].o);
-                else if (rec[e].kind == RES_SPAN)
-                    *out = res_sample<R>(a, q, c, rec[e].r, pend, cur);
-            }
-        }
+        if (wins && cur + 2 <= a.pt.nt) res_windows<R>(a, q, &win, cur + 1, cur + 1 <= src.last, false);
         if (ONE) {
             if ((int)threadIdx.x < items) res_v_item<R, H, STORE>(a, q, c, t0, kind, ck, slot, v_up, v_dn);
         } else {
@@ -842,8 +863,10 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_ac2d_fwd_res(const __grid_co
     if (a.fsurf) res_save_mirror<R>(a, q, c);
     __syncthreads();
     res_inject<R>(a, q, c, src, cur0 + q.n - 1);
-    const bool meet = near && cur0 + q.n <= src.last;
-    if ((taps || meet) && cur0 + q.n + 1 <= a.pt.nt) res_record(a, q, c.p, rec, cur0 + q.n, meet);
+    if (cur0 + q.n + 1 <= a.pt.nt) {
+        if (taps) res_record(a, c.p, rec, cur0 + q.n);
+        if (near && wins && cur0 + q.n <= src.last) res_windows<R>(a, q, &win, cur0 + q.n, true, true);
+    }
     res_save_state<R>(a, q, c);
     tick_last_block(a.d_step, a.pt.d_done, q.n);
 }
