@@ -1045,21 +1045,24 @@ struct Ac2dEngine : SsgBase {
         return store ? t * std::min(1.3, 1.0 + 0.05 * mc) : t;
     }
     using ResKernel = void (*)(Ac2dDev, Ac2dRes);
+    template <int RR, int H, bool ONE>
+    static ResKernel res_kernel_of(bool store, bool sample) {
+        return !store ? k_ac2d_fwd_res<RR, H, false, ONE, true>
+               : sample ? k_ac2d_fwd_res<RR, H, true, ONE, true> : k_ac2d_fwd_res<RR, H, true, ONE, false>;
+    }
+    // (segments that store record traces in the forward, not when recomputed)
     template <int RR>
-    static ResKernel res_kernel(int H, bool store, bool one) {
-        if (RR == 4 && H == 4)
-            return store ? (one ? k_ac2d_fwd_res<4, 4, true, true> : k_ac2d_fwd_res<4, 4, true, false>)
-                         : (one ? k_ac2d_fwd_res<4, 4, false, true> : k_ac2d_fwd_res<4, 4, false, false>);
-        return store ? (one ? k_ac2d_fwd_res<RR, 2, true, true> : k_ac2d_fwd_res<RR, 2, true, false>)
-                     : (one ? k_ac2d_fwd_res<RR, 2, false, true> : k_ac2d_fwd_res<RR, 2, false, false>);
+    static ResKernel res_kernel(int H, bool one, bool store, bool sample) {
+        if (RR == 4 && H == 4) return one ? res_kernel_of<4, 4, true>(store, sample) : res_kernel_of<4, 4, false>(store, sample);
+        return one ? res_kernel_of<RR, 2, true>(store, sample) : res_kernel_of<RR, 2, false>(store, sample);
     }
     template <int RR>
     const ResPlan& res_plan(int S) {
         auto it = res_plans.find(S);
         if (it != res_plans.end()) return it->second;
         ResPlan best;
-        for (int v = 0; v < 8; ++v) {
-            auto f = res_kernel<RR>(v & 1 ? 4 : 2, v & 2, v & 4);
+        for (int v = 0; v < 16; ++v) {
+            auto f = res_kernel<RR>(v & 1 ? 4 : 2, v & 2, v & 4, v & 8);
             OWL_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
             OWL_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RES_SMEM));
         }
@@ -1093,7 +1096,7 @@ struct Ac2dEngine : SsgBase {
             cfg.blockDim = dim3(p.threads);
             cfg.dynamicSmemBytes = p.smem;
             int slots = 0;
-            if (cudaOccupancyMaxActiveClusters(&slots, res_kernel<RR>(p.H, true, p.one), &cfg) != cudaSuccess || slots < 1) {
+            if (cudaOccupancyMaxActiveClusters(&slots, res_kernel<RR>(p.H, p.one, true, true), &cfg) != cudaSuccess || slots < 1) {
                 (void)cudaGetLastError();
                 continue;
             }
@@ -1140,12 +1143,10 @@ struct Ac2dEngine : SsgBase {
         Ac2dDev a = dev(S);
         Ac2dRes q = p.q;
         q.n = n;
-        q.smp = kind != 1;
         q.inj_last = inj_last.p;
         q.org = rec_org.p;
-        q.fac = windows && q.smp ? rec_fac.p : nullptr;
-        const bool store = kind == 1 || kind == 3;
-        const ResKernel k = res_kernel<RR>(p.H, store, p.one);
+        q.fac = windows && kind != 1 ? rec_fac.p : nullptr;
+        const ResKernel k = res_kernel<RR>(p.H, p.one, kind == 1 || kind == 3, kind != 1);
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;

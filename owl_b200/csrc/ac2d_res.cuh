@@ -42,7 +42,6 @@ struct Ac2dRes {
     int XG, XP;       // four-cell groups of a row; shared row pitch (4 XG + 2 R floats)
     int GL, GR, GN;   // groups g < GL or g >= GR hold x-PML cells; GN of them
     int zlo;          // storage row of the first resident row (the surface row with a free surface)
-    int smp;          // record receivers
     int zb[RES_MAXC + 1];  // first resident row of each CTA, relative to zlo
     const int* inj_last;   // per shot: last step (1-based) with a nonzero amplitude
     const int2* org;       // traces of several taps: storage (x, z) of the window's first tap
@@ -352,19 +351,18 @@ __device__ __noinline__ int res_find_receivers(const Ac2dDev& a, const Ac2dRes& 
     __syncthreads();
     const Ac2dPt& t = a.pt;
     bool near = false;
-    if (q.smp)
-        for (int r = t.rec_ptr[c.s] + threadIdx.x; r < t.rec_ptr[c.s + 1]; r += blockDim.x) {
-            const int j = t.smp.ptr[r], n = t.smp.ptr[r + 1] - j;
-            if (n == 0) continue;  // no taps: the trace is zero
-            const int2 g = n == 1 ? make_int2(0, 0) : q.org[r];
-            near |= n > 1 && ac2d_inj_near(t, c.s, 1, g.x, g.x + BOX_W, g.y, g.y + BOX_W);
-            int l = (n == 1 ? (int)(t.smp.off[j] / a.pitch) : g.y + BOX_W / 2) - q.zlo;
-            l = min(max(l, 0), q.zb[q.C] - 1) - c.l0;
-            if (l >= 0 && l < c.nr) {
-                const int k = atomicAdd(list, 1);
-                if (k < 2 * (int)blockDim.x) list[1 + k] = r;
-            }
+    for (int r = t.rec_ptr[c.s] + threadIdx.x; r < t.rec_ptr[c.s + 1]; r += blockDim.x) {
+        const int j = t.smp.ptr[r], n = t.smp.ptr[r + 1] - j;
+        if (n == 0) continue;  // no taps: the trace is zero
+        const int2 g = n == 1 ? make_int2(0, 0) : q.org[r];
+        near |= n > 1 && ac2d_inj_near(t, c.s, 1, g.x, g.x + BOX_W, g.y, g.y + BOX_W);
+        int l = (n == 1 ? (int)(t.smp.off[j] / a.pitch) : g.y + BOX_W / 2) - q.zlo;
+        l = min(max(l, 0), q.zb[q.C] - 1) - c.l0;
+        if (l >= 0 && l < c.nr) {
+            const int k = atomicAdd(list, 1);
+            if (k < 2 * (int)blockDim.x) list[1 + k] = r;
         }
+    }
     __syncthreads();
     const int count = list[0];
     for (int e = 0; e < 2; ++e) {
@@ -786,8 +784,8 @@ __device__ __forceinline__ void res_v_item(const Ac2dDev& a, const Ac2dRes& q, c
     if (t.uv | t.dv) res_push<R, H>(t, c.vz, q.XP, t.uv, t.dv, up, dn);
 }
 
-// ONE: every item of the CTA has its own thread
-template <int R, int H, bool STORE, bool ONE>
+// ONE: every item of the CTA has its own thread; SMP: traces are recorded
+template <int R, int H, bool STORE, bool ONE, bool SMP>
 __global__ void __launch_bounds__(RES_THREADS, 1) k_ac2d_fwd_res(const __grid_constant__ Ac2dDev a,
                                                                  const __grid_constant__ Ac2dRes q) {
     extern __shared__ __align__(16) float res_sm[];
@@ -796,10 +794,15 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_ac2d_fwd_res(const __grid_co
     const int cur0 = *a.d_step;
     ResRec found[2];
     ResWin win;
-    const int has = res_find_receivers<R>(a, q, found, &win);
-    const ResRec rec[2] = {found[0], found[1]};
+    int has = 0;
+    if (SMP) has = res_find_receivers<R>(a, q, found, &win);
+    ResRec rec[2];
+    if (SMP) {
+        rec[0] = found[0];
+        rec[1] = found[1];
+    }
     const bool taps = has & RES_HAS_TAPS, near = has & RES_HAS_NEAR;
-    const bool wins = win.kind[0] != RES_NONE || win.kind[1] != RES_NONE;  // the thread has traces of several taps
+    const bool wins = SMP && (win.kind[0] != RES_NONE || win.kind[1] != RES_NONE);  // the thread has traces of several taps
     ResSrc src;
     res_find_source<R>(a, q, c, near, src);
     const float* amp = a.pt.amp + (size_t)src.it * a.pt.nt;
@@ -848,7 +851,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_ac2d_fwd_res(const __grid_co
         cluster_arrive();
         if (cur + 1 <= src.last && src.nit > 0) src.A = __ldg(amp + cur);
         cluster_wait();
-        if (wins && cur + 2 <= a.pt.nt) res_windows<R>(a, q, &win, cur + 1, cur + 1 <= src.last, false);
+        if (SMP && wins && cur + 2 <= a.pt.nt) res_windows<R>(a, q, &win, cur + 1, cur + 1 <= src.last, false);
         if (ONE) {
             if ((int)threadIdx.x < items) res_v_item<R, H, STORE>(a, q, c, t0, kind, ck, slot, v_up, v_dn);
         } else {
@@ -863,7 +866,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_ac2d_fwd_res(const __grid_co
     if (a.fsurf) res_save_mirror<R>(a, q, c);
     __syncthreads();
     res_inject<R>(a, q, c, src, cur0 + q.n - 1);
-    if (cur0 + q.n + 1 <= a.pt.nt) {
+    if (SMP && cur0 + q.n + 1 <= a.pt.nt) {
         if (taps) res_record(a, c.p, rec, cur0 + q.n);
         if (near && wins && cur0 + q.n <= src.last) res_windows<R>(a, q, &win, cur0 + q.n, true, true);
     }
