@@ -3,30 +3,33 @@
 //
 // A step kernel reads and writes a shot's whole state through L2 twice a step
 // and pays a launch boundary for each of its passes. Here one thread-block
-// cluster owns one shot for all n steps of a launch: its C CTAs (C = 1 .. 16)
-// hold consecutive rows of p, vx, vz and the CFS-PML memories in shared memory
+// cluster owns one shot for all n steps of a launch: its C CTAs (C = 1,
+// 2, 4, 8 or 16) hold consecutive rows of p, vx, vz and the CFS-PML memories in shared memory
 // (with the coefficients about 3.1 MB for a 441 x 241 grid, 16 CTAs), each row
 // whole, so that x neighbours are always local and only R boundary rows cross
 // to the neighbouring CTAs, written into their halo rows (distributed shared
 // memory) by the thread that computes them. A step is two phases, each ended by
 // the cluster's hardware barrier (0.25 us; no polling):
-//   P: the pending explosion taps of the step before, then
+//   P: the pending explosion taps of the step before, the receivers on one node, then
 //      p -= dtbk (dx vx + dz vz)                      -> p rows to both neighbours
-//   V: vx -= dtbx dx p, vz -= dtbz dz p; receivers    -> vz rows to both neighbours
+//   V: vx -= dtbx dx p, vz -= dtbz dz p               -> vz rows to both neighbours
+//      and the receivers between nodes, from their window of 9 x 9 nodes
 // Global memory sees only the traces, the stored stencil terms of the STORE
 // variant, and the state and coefficients once a launch.
 //
 // A thread owns H rows x 4 cells: the z arms come from one column window of
 // 2R - 1 + H float4 rows held in registers, the x arms from R / 2 + 1 float4
 // loads per row, the arithmetic is packed two cells per instruction where the
-// operands lie in pairs. What bounds it: shared-memory reads (about 20 float4 per
-// four cells and step, 5.3 k of the 9.6 k cycles of a step of a 441 x 241 grid),
-// instruction issue (0.4 per cycle and scheduler) and the two barriers (1.3 k
-// cycles). Measured on B200, us per step against the step launches (CUDA graph):
-// one shot 441 x 241 5.0 / 8.8, seven 5.3 / 13.2, 32 25.7 / 35.7; one shot
-// 181 x 131 2.7 / 8.2. Rows of the coefficients in registers or read through L2
-// each step (spills and L1 misses: 8.1 us), and one code path with tests for the
-// PML per row (5.1 us with a third more instructions), measured slower.
+// operands lie in pairs. What bounds it (counters of seven shots of 401 x 201, 16
+// CTAs each): shared-memory wavefronts, 60 % of the cycles of the SMs in use and 66 %
+// of the busiest; the barriers, a third of a warp's time (CTA barrier 19 %, the
+// release before the cluster's 14 %); issue, 0.31 per cycle and scheduler. The storing
+// variant adds its stores to HBM (1.17 TB/s). Measured on B200, us per step against
+// the step launches (CUDA graph), 401 x 201: 8 shots 10.5 / 16.1, 32 26.0 / 34.5,
+// 64 52.8 / 82.6; one shot of 151 x 101 2.4 / 8.5. Rows of the coefficients in
+// registers or read through L2 each step (spills and L1 misses: 8.1 us a wave), and one
+// code path with tests for the PML per row (5.1 us with a third more instructions),
+// measured slower.
 //
 // Per cell the arithmetic is that of the one-cell step kernels (ac2d.cu), in the
 // same order and rounding: traces, stored terms and states equal theirs to the bit.
