@@ -154,7 +154,6 @@ struct DevBuf {
 // ----------------------------------------------------------------------------
 struct Tap {
     int field;   // field slot within the medium's state (e.g. 0 = p, 1 = vx, 2 = vz)
-    int shot;    // shot index inside the batch
     int64_t off; // offset inside one shot's field (z * pitch + x)
     float w;     // weight
     int item;    // owning item for scatter tables (receiver / source index)
@@ -162,12 +161,11 @@ struct Tap {
 
 struct HostCSR {
     std::vector<int> ptr{0};
-    std::vector<int> field, shot, item;
+    std::vector<int> field, item;
     std::vector<long long> off;
     std::vector<float> w;
     void push(const Tap& t) {
         field.push_back(t.field);
-        shot.push_back(t.shot);
         item.push_back(t.item);
         off.push_back(t.off);
         w.push_back(t.w);
@@ -185,22 +183,23 @@ struct alignas(16) TapRec {
 };
 
 struct DevCSR {
-    DevBuf<int> ptr, field, shot, item;
+    DevBuf<int> ptr, field, item;
     DevBuf<long long> off;
     DevBuf<float> w;
     DevBuf<TapRec> tap;
     int nitems = 0, ntaps = 0;
-    // by_item: the packed taps carry the item instead of the field
-    void upload(const HostCSR& h, cudaStream_t s, bool by_item = false) {
+    // scatter: a scatter table, whose packed taps carry the item instead of the
+    // field; split: the parts by themselves too, for point work inside stencil kernels
+    void upload(const HostCSR& h, cudaStream_t s, bool scatter, bool split) {
         nitems = h.nitems();
         ntaps = h.ntaps();
         std::vector<TapRec> t(ntaps);
-        for (int j = 0; j < ntaps; ++j) t[j] = TapRec{h.off[j], by_item ? h.item[j] : h.field[j], h.w[j]};
+        for (int j = 0; j < ntaps; ++j) t[j] = TapRec{h.off[j], scatter ? h.item[j] : h.field[j], h.w[j]};
         tap.upload(t.data(), t.size(), s);
         ptr.upload(h.ptr.data(), h.ptr.size(), s);
-        field.upload(h.field.data(), h.field.size(), s);
-        shot.upload(h.shot.data(), h.shot.size(), s);
-        item.upload(h.item.data(), h.item.size(), s);
+        if (scatter) field.upload(h.field.data(), h.field.size(), s);
+        if (!split) return;
+        if (scatter) item.upload(h.item.data(), h.item.size(), s);
         off.upload(h.off.data(), h.off.size(), s);
         w.upload(h.w.data(), h.w.size(), s);
     }
@@ -209,17 +208,16 @@ struct DevCSR {
 // device view of a CSR table
 struct CSRView {
     const int* ptr;
-    const int* field;
-    const int* shot;
-    const int* item;
-    const long long* off;
-    const float* w;
+    const int* field;  // scatter tables
+    const int* item;   // scatter tables, split
+    const long long* off;  // split
+    const float* w;        // split
     const TapRec* tap;
     int nitems;
 };
 
 inline CSRView view(const DevCSR& d) {
-    return CSRView{d.ptr.p, d.field.p, d.shot.p, d.item.p, d.off.p, d.w.p, d.tap.p, d.nitems};
+    return CSRView{d.ptr.p, d.field.p, d.item.p, d.off.p, d.w.p, d.tap.p, d.nitems};
 }
 
 // FD coefficients of the optimised staggered scheme (src/lib/module_fdcoef.f90:23-30, 59-62)

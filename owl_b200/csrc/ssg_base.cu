@@ -390,7 +390,7 @@ void SsgBase::build_tables(int S, const owl_shot* shots, bool need_sct) {
                 for (const TapPt& t : taps) {
                     if (t.w == 0.f) continue;
                     OWL_CHECK(in_wavefield(t.i, t.j, t.k), OWL_ERR_INVALID, "source tap outside the padded grid");
-                    hinj.push(Tap{t.field, s, soff(t.i, t.j, t.k), t.w, 0});
+                    hinj.push(Tap{t.field, soff(t.i, t.j, t.k), t.w, 0});
                     bi = std::min(bi, t.i); bj = std::min(bj, t.j); bk = std::min(bk, t.k);
                     if (bf < 0) bf = t.field;
                     if (bf != t.field) fuse = false;
@@ -439,7 +439,7 @@ void SsgBase::build_tables(int S, const owl_shot* shots, bool need_sct) {
                     for (const TapPt& t : taps) {
                         if (t.w == 0.f) continue;
                         OWL_CHECK(in_wavefield(t.i, t.j, t.k), OWL_ERR_INVALID, "receiver tap outside the padded grid");
-                        hsmp.push(Tap{t.field, s, soff(t.i, t.j, t.k), t.w, rg});
+                        hsmp.push(Tap{t.field, soff(t.i, t.j, t.k), t.w, rg});
                         fuse &= fuse_tap_ok(t.field, t.i + pr - 1, dim == 3 ? t.j + pr - 1 : 0, t.k + pr - 1, true);
                         if (need_sct) {
                             mapped.clear();
@@ -457,7 +457,7 @@ void SsgBase::build_tables(int S, const owl_shot* shots, bool need_sct) {
             }
         }
         for (auto& kv : cells) {
-            for (auto& e : kv.second) hsct.push(Tap{kv.first.first, s, kv.first.second, e.second, e.first});
+            for (auto& e : kv.second) hsct.push(Tap{kv.first.first, kv.first.second, e.second, e.first});
             hsct.close_item();
         }
         for (int comp = 0; comp < ncomp; ++comp) h_gather_ptr.push_back(rtot + (comp + 1) * sh.nrec);
@@ -493,9 +493,10 @@ void SsgBase::build_tables(int S, const owl_shot* shots, bool need_sct) {
     }
     nb_rec = ctas(mr);
     nb_sct = ctas(ms);
-    inj.upload(hinj, stream);
-    smp.upload(hsmp, stream);
-    sct.upload(hsct, stream, true);
+    const bool split = fuse_supported();
+    inj.upload(hinj, stream, false, false);
+    smp.upload(hsmp, stream, false, split);
+    sct.upload(hsct, stream, true, split);
     inj_shot_ptr.upload(hinj_ptr.data(), hinj_ptr.size(), stream);
     rec_shot_ptr.upload(hrec_ptr.data(), hrec_ptr.size(), stream);
     sct_shot_ptr.upload(hsct_ptr.data(), hsct_ptr.size(), stream);
@@ -630,8 +631,8 @@ void SsgBase::run_steps(int kind, int n, int S, const PointDev& q, bool graph) {
     std::vector<uintptr_t> sig = {(uintptr_t)n, (uintptr_t)S, (uintptr_t)spt_f, (uintptr_t)spt_a, (uintptr_t)tz_f,
                                   (uintptr_t)tz_a, (uintptr_t)cur_k, (uintptr_t)tile_x, (uintptr_t)st.p,
                                   (uintptr_t)ad.p, (uintptr_t)Sbuf.p, (uintptr_t)G.p, (uintptr_t)rec.p,
-                                  (uintptr_t)res.p, (uintptr_t)q.src_adj, (uintptr_t)inj.ptr.p, (uintptr_t)inj.w.p,
-                                  (uintptr_t)inj.off.p, (uintptr_t)smp.ptr.p, (uintptr_t)smp.w.p, (uintptr_t)smp.off.p,
+                                  (uintptr_t)res.p, (uintptr_t)q.src_adj, (uintptr_t)inj.ptr.p, (uintptr_t)smp.ptr.p,
+                                  (uintptr_t)sct.item.p, (uintptr_t)smp.w.p, (uintptr_t)smp.off.p,
                                   (uintptr_t)sct.ptr.p, (uintptr_t)sct.w.p, (uintptr_t)sct.off.p, (uintptr_t)inj.tap.p,
                                   (uintptr_t)smp.tap.p, (uintptr_t)sct.tap.p, (uintptr_t)sct.field.p, (uintptr_t)amp.p,
                                   (uintptr_t)inj_shot_ptr.p, (uintptr_t)rec_shot_ptr.p, (uintptr_t)sct_shot_ptr.p,
