@@ -28,8 +28,9 @@ namespace owl {
 // the taps of a trace are read eight at a time (their fields in parallel, the
 // sum in tap order). One thread per trace keeps it to one round. On the 16-shot
 // elastic 2D line (602 traces of 9 taps per shot) a time step went from 102.5 to
-// 95.1 us, in the 8-shot gradient from 68.6 to 62.8 ms per 800 steps, against
-// one CTA per shot reading tap by tap.
+// 94.3 us, in the 8-shot gradient from 68.0 to 61.0 ms per 800 steps, against
+// one CTA per shot reading tap by tap (62.7 ms with the source-side adjoint's taps
+// one after another, which cost a 3D gradient 10 us a step over the tables before).
 constexpr int POINT_TAPS = 8;
 
 // acc + sum of the taps [j, j1) of one trace, in order; `first` holds the taps
@@ -44,7 +45,8 @@ __device__ __forceinline__ void load_taps(const TapRec* __restrict__ tap, int j,
             t[q].w = __int_as_float(v.w);
         }
 }
-__device__ __forceinline__ float sample_taps(const PointDev& a, long long so, int j, int j1, TapRec (&t)[POINT_TAPS]) {
+__device__ __forceinline__ float sample_taps(const PointDev& a, const TapRec* __restrict__ tap, long long so, int j, int j1,
+                                             TapRec (&t)[POINT_TAPS]) {
     float acc = 0.f;
     while (j < j1) {
         float f[POINT_TAPS];
@@ -56,7 +58,7 @@ __device__ __forceinline__ float sample_taps(const PointDev& a, long long so, in
         for (int q = 0; q < POINT_TAPS; ++q)
             if (j + q < j1) acc = acc + f[q] * t[q].w;
         j += POINT_TAPS;
-        if (j < j1) load_taps(a.smp.tap, j, j1, t);
+        if (j < j1) load_taps(tap, j, j1, t);
     }
     return acc;
 }
@@ -99,7 +101,7 @@ __global__ void __launch_bounds__(256) k_point_fwd(const __grid_constant__ Point
     const int tr = (mode & PT_NEXT) ? t + 1 : t;
     if (tr <= a.nt) {
         while (r < rend) {
-            a.rec[(size_t)(tr - 1) * a.rtot + r] = sample_taps(a, so, j0, j1, t0);
+            a.rec[(size_t)(tr - 1) * a.rtot + r] = sample_taps(a, a.smp.tap, so, j0, j1, t0);
             r += step;
             if (r < rend) {
                 j0 = __ldg(a.smp.ptr + r);
@@ -165,12 +167,9 @@ __global__ void __launch_bounds__(256) k_point_adj(const __grid_constant__ Point
     const int ts = (mode & PA_SRC) ? t - 1 : t;
     if ((mode & (PA_SRC | PA_SRC_NOW)) && blockIdx.y == 0 && a.src_adj && ts >= 1) {
         for (int i = a.inj_shot_ptr[s] + threadIdx.x; i < a.inj_shot_ptr[s + 1]; i += blockDim.x) {
-            float acc = 0.f;
-            for (int j = a.inj.ptr[i]; j < a.inj.ptr[i + 1]; ++j) {
-                const TapRec q = a.inj.tap[j];
-                acc = acc + __ldcg(a.fld[q.fi] + so + q.off) * q.w;
-            }
-            a.src_adj[(size_t)i * a.nt + (ts - 1)] = acc;
+            const int k0 = a.inj.ptr[i], k1 = a.inj.ptr[i + 1];
+            load_taps(a.inj.tap, k0, k1, t0);
+            a.src_adj[(size_t)i * a.nt + (ts - 1)] = sample_taps(a, a.inj.tap, so, k0, k1, t0);
         }
     }
     if (mode & PA_TICK) tick_last_block(a.d_step, a.d_done, -1);
