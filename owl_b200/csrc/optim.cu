@@ -196,10 +196,18 @@ __global__ void __launch_bounds__(256) k_cg_apply(long long n, const double* __r
         srch[i] = (float)(-(double)g[i] + beta * (double)prev[i]);
 }
 
-// (r may be g)
-__global__ void k_negate(long long n, const float* g, float* r) {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        r[i] = -g[i];
+// (r may be g: LB_CELLS cells a thread at once, their reads ahead of their writes)
+__global__ void __launch_bounds__(256) k_negate(long long n, const float* g, float* r) {
+    const long long step = (long long)gridDim.x * blockDim.x;
+    for (long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += LB_CELLS * step) {
+        float v[LB_CELLS];
+#pragma unroll
+        for (int e = 0; e < LB_CELLS; ++e)
+            if (i0 + e * step < n) v[e] = g[i0 + e * step];
+#pragma unroll
+        for (int e = 0; e < LB_CELLS; ++e)
+            if (i0 + e * step < n) r[i0 + e * step] = -v[e];
+    }
 }
 
 // one axis of a separable filter: field (n1, n2, n3), axis stride `st`, length `len`.
